@@ -54,6 +54,21 @@ __device__ __forceinline__ float2 *psi_pairs(const fdtd_dev &d, int a) {
   return reinterpret_cast<float2 *>(d.psi[a]);
 }
 
+// psi pair addresses of a cell (H and E share the slab layouts; px, py, pz:
+// the cell's slab positions).
+__device__ __forceinline__ int psi_x_pos(const fdtd_dev &d, int px) {
+  return px < d.p ? px : px + fdtd_psi_x_off(d.I, d.p);
+}
+__device__ __forceinline__ float2 *psi_at_y(const fdtd_dev &d, int a, int i, int py, int k) {
+  return psi_pairs(d, a) + (i + (py + k * 2 * (int64_t)d.p) * d.Ip);
+}
+__device__ __forceinline__ float2 *psi_at_x(const fdtd_dev &d, int a, int px, int j, int k) {
+  return psi_pairs(d, a) + (psi_x_pos(d, px) + (j + k * (int64_t)d.J) * fdtd_psi_x_pitch(d.I, d.p));
+}
+__device__ __forceinline__ float2 *psi_at_z(const fdtd_dev &d, int a, int i, int j, int pz) {
+  return psi_pairs(d, a) + (i + j * (int64_t)d.Ip + pz * d.plane);
+}
+
 // Slab position of index v in a CPML of thickness p on an axis of length n.
 // H cells: low side [0,p) -> v, high side [n-p, n-2] -> v-n+2p
 // (src/gpu.h:615-617, :654-656, :698-700).
@@ -303,17 +318,6 @@ __device__ __forceinline__ void h_corr_z(const fdtd_dev &d, int pz, float2 ps, f
   *dst = make_float2(v0, v1);
 }
 
-// psi pair addresses of a cell (H and E share the slab layouts).
-__device__ __forceinline__ float2 *psi_at_y(const fdtd_dev &d, int a, int i, int py, int k) {
-  return psi_pairs(d, a) + (i + py * (int64_t)d.I + k * 2 * (int64_t)d.p * d.I);
-}
-__device__ __forceinline__ float2 *psi_at_x(const fdtd_dev &d, int a, int px, int j, int k) {
-  return psi_pairs(d, a) + (px + j * 2 * (int64_t)d.p + k * 2 * (int64_t)d.p * d.J);
-}
-__device__ __forceinline__ float2 *psi_at_z(const fdtd_dev &d, int a, int i, int j, int pz) {
-  return psi_pairs(d, a) + (i + j * (int64_t)d.I + pz * d.IJ);
-}
-
 // New H of one cell from its old H and the six forward E differences:
 // curl (gpu.h:575-602), TF/SF, CPML Y (gpu.h:644-685), X (:604-642),
 // Z (:687-725).  px/py/pz: H-slab positions (-1 outside).  C: the cell's
@@ -335,15 +339,16 @@ __device__ __forceinline__ void update_h_cell(const fdtd_dev &d, const HCoef &C,
   if (mode) tfsf_h(d, mode, inc, i, j, k, hx, hy, hz, C.hex, C.hey, C.hez);
   if (PML) {
     // Each psi pair belongs to one cell, so all of the cell's pairs are
-    // loaded before its first psi store: one memory round trip.
-    const int64_t I = d.I, J = d.J, pj = 2 * (int64_t)d.p;
-    float2 *Y = psi_pairs(d, PSI_HY) + (i + py * I + k * pj * I);
-    float2 *X = psi_pairs(d, PSI_HX) + (px + j * pj + k * pj * J);
-    float2 *Z = psi_pairs(d, PSI_HZ) + (i + j * I + pz * d.IJ);
+    // loaded before its first psi store: one memory round trip.  They come
+    // from L2: no line is read twice, and in the multi-step kernel another
+    // SM may have written it.
+    float2 *Y = psi_at_y(d, PSI_HY, i, py, k);
+    float2 *X = psi_at_x(d, PSI_HX, px, j, k);
+    float2 *Z = psi_at_z(d, PSI_HZ, i, j, pz);
     float2 y = make_float2(0.f, 0.f), x = y, z = y;
-    if (py >= 0) y = *Y;
-    if (px >= 0) x = *X;
-    if (pz >= 0) z = *Z;
+    if (py >= 0) y = __ldcg(Y);
+    if (px >= 0) x = __ldcg(X);
+    if (pz >= 0) z = __ldcg(Z);
     if (py >= 0) h_corr_y(d, py, y, Y, dEz_y, dEx_y, hx, hz, C.hex, C.hez);
     if (px >= 0) h_corr_x_bc(d, xb[px], xc[px], x, X, dEz_x, dEy_x, hy, hz, C.hey, C.hez);
     if (pz >= 0) h_corr_z(d, pz, z, Z, dEy_z, dEx_z, hx, hy, C.hex, C.hey);
@@ -397,15 +402,10 @@ __device__ __forceinline__ void e_corr_x_bc(const fdtd_dev &d, float b, float c,
   ez = ez + C.ezh * v1 * dx;
   *dst = make_float2(v0, v1);
 }
-__device__ __forceinline__ void e_corr_x(const fdtd_dev &d, int px, float2 ps, float2 *dst,
-                                         const Coef6 &C, float hz, float hz_im, float hy,
-                                         float hy_im, float &ey, float &ez) {
-  e_corr_x_bc(d, d.bE[px], d.cE[px], ps, dst, C, hz, hz_im, hy, hy_im, ey, ez);
-}
-
 // New E of one cell: curl with the reference's guards (gpu.h:727-763),
 // TF/SF, CPML Y (gpu.h:790-827), Z (:829-868), X (:765-788), then the
-// current source (gpu.h:55-82) when `cur` is set.
+// current source (gpu.h:55-82) when `cur` is set.  xb, xc: the E grading
+// tables for the X axis (see update_h_cell).
 template <bool CURL, bool PML>
 __device__ __forceinline__ void update_e_cell(const fdtd_dev &d, int mode, const float *inc,
                                               int cur_mode, float cur_src, bool cur, int i,
@@ -413,7 +413,8 @@ __device__ __forceinline__ void update_e_cell(const fdtd_dev &d, int mode, const
                                               const Coef6 &C, float &ex, float &ey, float &ez,
                                               float hx, float hy, float hz, float hz_jm,
                                               float hx_jm, float hz_im, float hy_im,
-                                              float hx_km, float hy_km) {
+                                              float hx_km, float hy_km, const float *xb,
+                                              const float *xc) {
   const float dx = d.dx;
   if (CURL) {
     if (j != 0 && k != 0) ex = C.exe * ex + C.exh * (+(hz - hz_jm) - (hy - hy_km));
@@ -423,23 +424,58 @@ __device__ __forceinline__ void update_e_cell(const fdtd_dev &d, int mode, const
   if (mode) tfsf_e(d, mode, inc, i, j, k, C.exh, C.eyh, C.ezh, ex, ey, ez);
   if (PML) {
     // all psi pairs of the cell first (see update_h_cell)
-    const int64_t I = d.I, J = d.J, pj = 2 * (int64_t)d.p;
-    float2 *Y = psi_pairs(d, PSI_EY) + (i + py * I + k * pj * I);
-    float2 *Z = psi_pairs(d, PSI_EZ) + (i + j * I + pz * d.IJ);
-    float2 *X = psi_pairs(d, PSI_EX) + (px + j * pj + k * pj * J);
+    float2 *Y = psi_at_y(d, PSI_EY, i, py, k);
+    float2 *Z = psi_at_z(d, PSI_EZ, i, j, pz);
+    float2 *X = psi_at_x(d, PSI_EX, px, j, k);
     float2 y = make_float2(0.f, 0.f), z = y, x = y;
-    if (py >= 0) y = *Y;
-    if (pz >= 0) z = *Z;
-    if (px >= 0) x = *X;
+    if (py >= 0) y = __ldcg(Y);
+    if (pz >= 0) z = __ldcg(Z);
+    if (px >= 0) x = __ldcg(X);
     if (py >= 0) e_corr_y(d, py, y, Y, C, hz, hz_jm, hx, hx_jm, ex, ez);
     if (pz >= 0) e_corr_z(d, pz, z, Z, C, hy, hy_km, hx, hx_km, ex, ey);
-    if (px >= 0) e_corr_x(d, px, x, X, C, hz, hz_im, hy, hy_im, ey, ez);
+    if (px >= 0) e_corr_x_bc(d, xb[px], xc[px], x, X, C, hz, hz_im, hy, hy_im, ey, ez);
   }
   if (cur) {  // E -= Ce?h * source * dx / dx / dx
     if (cur_mode == 1) ex = ex - C.exh * cur_src * dx / dx / dx;
     else if (cur_mode == 2) ey = ey - C.eyh * cur_src * dx / dx / dx;
     else ez = ez - C.ezh * cur_src * dx / dx / dx;
   }
+}
+
+// ------------------------------------------- oblique plane wave (mode 5)
+
+// Window value at coordinate x (linear interpolation between nodes).
+__device__ __forceinline__ float ob_interp(const float *row, float x, int w) {
+  int m = (int)floorf(x);
+  m = m < 0 ? 0 : (m > w - 2 ? w - 2 : m);
+  const float f = x - (float)m;
+  return row[m] + f * (row[m + 1] - row[m]);
+}
+
+// Window coordinate of a point (px, py, pz) in cells: ob_rho 1D nodes per
+// cell of distance along k.
+__device__ __forceinline__ float ob_coord(const fdtd_dev &d, float px, float py, float pz) {
+  const float s = d.ob_k[0] * (px - (float)d.ob_r0[0]) + d.ob_k[1] * (py - (float)d.ob_r0[1]) +
+                  d.ob_k[2] * (pz - (float)d.ob_r0[2]);
+  return d.ob_x0 + d.ob_rho * s;
+}
+
+// One correction of E_ce from the face of axis A on the given side (0 low, 1
+// high): val +- c * h_ch * H1 of the H cell half a cell outside the face.
+template <int A, int CE>
+__device__ __forceinline__ float ob_e_corr(const fdtd_dev &d, const float *rowH, int x0, int x1,
+                                           int x2, int side, float c, float val) {
+  constexpr int CH = 3 - A - CE;            // the H component the face pairs with E_ce
+  constexpr bool T0 = CE == (A + 1) % 3;    // pair (E_u, H_v)
+  const int lo = A == 0 ? d.i0 : (A == 1 ? d.j0 : d.k0);
+  const int hi = A == 0 ? d.i1 : (A == 1 ? d.j1 : d.k1);
+  const int xa = side ? hi : lo - 1;        // the H cell outside the face
+  const float p0 = (float)(A == 0 ? xa : x0) + (CH != 0 ? 0.5f : 0.f);
+  const float p1 = (float)(A == 1 ? xa : x1) + (CH != 1 ? 0.5f : 0.f);
+  const float p2 = (float)(A == 2 ? xa : x2) + (CH != 2 ? 0.5f : 0.f);
+  const float inc = d.ob_h[CH] * ob_interp(rowH, ob_coord(d, p0, p1, p2) - 0.5f, d.ob_w);
+  const float t = c * inc;
+  return (T0 == (side == 0)) ? val + t : val - t;
 }
 
 }  // namespace fdtd

@@ -179,9 +179,9 @@ __device__ __forceinline__ void new_h(const fdtd_dev &d, const FusedParams &fp,
   }
   if (__any_sync(0xffffffffu, px >= 0 || py >= 0 || pz >= 0)) {
     // CPML Y, X, Z (the reference's launch order); all pairs loaded first
-    const int64_t Il = I, Jl = J, pj = 2 * (int64_t)p;
-    const int64_t iy = i + py * Il + h * pj * Il, ix = px + j * pj + h * pj * Jl;
-    const int64_t iz = i + j * Il + pz * d.IJ;
+    const int64_t iy = psi_at_y(d, PSI_HY, i, py, h) - psi_pairs(d, PSI_HY);
+    const int64_t ix = psi_at_x(d, PSI_HX, px, j, h) - psi_pairs(d, PSI_HX);
+    const int64_t iz = psi_at_z(d, PSI_HZ, i, j, pz) - psi_pairs(d, PSI_HZ);
     float2 sy = make_float2(0.f, 0.f), sx = sy, sz = sy;
     if (py >= 0) sy = reinterpret_cast<const float2 *>(fp.psi_h_old[0])[iy];
     if (px >= 0) sx = reinterpret_cast<const float2 *>(fp.psi_h_old[1])[ix];
@@ -396,7 +396,7 @@ __global__ void __launch_bounds__(NT, FDTD_FUSED_MIN_BLOCKS)
             if (act)
               update_e_cell<true, true>(d, 0, nullptr, 0, 0.f, false, i, j, h, -1, py, pz, C, ex,
                                         ey, ez, hx, hy, hz, hz_jm, hx_jm, hz_im, hy_im, hxm[c],
-                                        hym[c]);
+                                        hym[c], d.bE, d.cE);
           } else {
             ex = C.exe * ex + C.exh * (+(hz - hz_jm) - (hy - hym[c]));
             ey = C.eye * ey + C.eyh * (+(hx - hxm[c]) - (hz - hz_im));
@@ -459,7 +459,7 @@ __global__ void k_fix_e(const __grid_constant__ fdtd_dev d, const float *eox, co
     const float hz_im = d.f[5][n - 1], hy_im = d.f[4][n - 1];
     const float hx_km = d.f[3][n - d.plane], hy_km = d.f[4][n - d.plane];
     update_e_cell<true, false>(d, 0, nullptr, 0, 0.f, false, i, j, k, -1, -1, -1, C, ex, ey, ez,
-                               hx, hy, hz, hz_jm, hx_jm, hz_im, hy_im, hx_km, hy_km);
+                               hx, hy, hz, hz_jm, hx_jm, hz_im, hy_im, hx_km, hy_km, d.bE, d.cE);
     d.f[0][n] = ex;
     d.f[1][n] = ey;
     d.f[2][n] = ez;

@@ -95,6 +95,8 @@ typedef struct sim {
   float poly_m, alpha_m, sig_max, alpha_max, kappa_max;
   int32_t i0, i1, j0, j1, k0, k1;
   int64_t size_x, size_y, size_z;
+  int32_t pxp, pxo;              /* X psi rows (fdtd_psi_x_pitch, fdtd_psi_x_off) */
+  int64_t psi_x, psi_y, psi_z;   /* floats of one psi array per axis (padded rows) */
   /* host copies (reference: pinned arrays of setConst / setSource) */
   float *d_raw[6];      /* sigma_x,y,z, eps_x,y,z as UpdateMaterial gave them
                            (device, packed I*J*K); unset: the defaults */
@@ -112,7 +114,9 @@ typedef struct sim {
   /* device */
   cudaStream_t stream;
   cudaEvent_t ev[MAX_EVENTS];
-  float *d_f[6], *d_ce[6], *d_psi_pool, *d_psi[FDTD_NUM_PSI];
+  float *d_f[6]; /* one allocation, fstride values per field */
+  int64_t fstride;
+  float *d_ce[6], *d_psi_pool, *d_psi[FDTD_NUM_PSI];
   float *d_den_ex, *d_den_hx, *d_inc[4], *d_src, *d_probes, *d_mu[3];
   /* per-cell H coefficients (fdtd_set_magnetic): mode 1 arrays, 2 indexed */
   int32_t hcoef_mode;
@@ -135,6 +139,7 @@ typedef struct sim {
   int32_t coef_mode, num_mat;
   int use_tma, allow_compress;
   fdtd_maps maps[FDTD_NUM_TILES]; /* per tile geometry (1: also the batch's) */
+  fdtd_maps_flow wmaps[FDTD_FLOW_TILES];
   int32_t tile_h, tile_e;          /* the autotuner's geometries */
   int32_t zc_h, zc_e; /* tuned z-planes per TMA work item (0: heuristic) */
   uint64_t device_bytes;
@@ -158,10 +163,18 @@ typedef struct sim {
   float *d_fb[6], *d_psib_pool;
   fdtd_dev dev_b;
   fdtd_maps_fused fmaps[2];
-  int32_t zc_f, fused;
+  int32_t zc_f, fused, fused_forced; /* forced: FDTD_FUSED=1 */
   cudaGraphExec_t gexec_f;
   int gf_mode, gf_probes;
   unsigned long long gf_kernels;
+  /* many steps per launch (fdtd_flow.cu): the row counters, the steps they
+   * have counted since they were zeroed, the probes by z-plane, and the item
+   * geometry */
+  uint32_t *d_flow;
+  uint32_t flow_base;
+  int flow_zeroed;
+  int32_t flow_tile, flow_zc;
+  int32_t *d_pz, *d_pat, n_pat;     /* n_pat -1: a probe position it cannot serve */
 } sim;
 
 /* ------------------------------------------------------------ registry */
@@ -398,10 +411,10 @@ int fdtd_destroy(fdtd_handle h) {
   dfree(s->d_psib_pool);
   for (int a = 0; a < 6; ++a) {
     dfree(s->d_fb[a]);
-    dfree(s->d_f[a]);
     dfree(s->d_ce[a]);
     dfree(s->d_raw[a]);
   }
+  dfree(s->d_f[0]);
   free(s->shapes);
   for (int a = 0; a < 4; ++a) dfree(s->d_inc[a]);
   dfree(s->d_ob[0]);
@@ -424,6 +437,9 @@ int fdtd_destroy(fdtd_handle h) {
   dfree(s->d_hrep);
   dfree(s->d_hid);
   dfree(s->d_hcnt);
+  dfree(s->d_flow);
+  dfree(s->d_pz);
+  dfree(s->d_pat);
   free(s->h_src);
   free(s->h_probe_idx);
   free(s->h_den_ex);
@@ -543,6 +559,11 @@ int fdtd_set_const(fdtd_handle h, const float freqRes[3], const int32_t timeDim[
   s->size_x = (int64_t)p * J * K;
   s->size_y = (int64_t)I * p * K;
   s->size_z = (int64_t)I * J * p;
+  s->pxp = fdtd_psi_x_pitch(I, p);
+  s->pxo = fdtd_psi_x_off(I, p);
+  s->psi_x = 2 * (int64_t)s->pxp * J * K;
+  s->psi_y = 2 * 2 * (int64_t)p * s->Ip * K;
+  s->psi_z = 2 * 2 * (int64_t)p * s->plane;
   s->init_const = 1;
   return FDTD_OK;
 }
@@ -724,8 +745,8 @@ static void fused_refresh(sim *s) {
   s->dev_b = s->dev;
   for (int a = 0; a < 6; ++a) s->dev_b.f[a] = s->d_fb[a];
   s->dev_b.psi[PSI_HY] = s->d_psib_pool;
-  s->dev_b.psi[PSI_HX] = s->d_psib_pool + 4 * s->size_y;
-  s->dev_b.psi[PSI_HZ] = s->d_psib_pool + 4 * (s->size_y + s->size_x);
+  s->dev_b.psi[PSI_HX] = s->d_psib_pool + s->psi_y;
+  s->dev_b.psi[PSI_HZ] = s->d_psib_pool + s->psi_y + s->psi_x;
   if (fdtdk_make_maps_fused(&s->dev, &s->fmaps[0])) s->fmaps[0].valid = 0;
   if (fdtdk_make_maps_fused(&s->dev_b, &s->fmaps[1])) s->fmaps[1].valid = 0;
 }
@@ -916,7 +937,7 @@ static int upload_coefficients(sim *s) {
 static int zero_state(sim *s) {
   const size_t bytes = (size_t)s->cells * sizeof(float);
   for (int a = 0; a < 6; ++a) CU(cudaMemsetAsync(s->d_f[a], 0, bytes, s->stream));
-  const size_t psi_total = (size_t)(4 * 2 * (s->size_x + s->size_y + s->size_z)) * sizeof(float);
+  const size_t psi_total = (size_t)(2 * (s->psi_x + s->psi_y + s->psi_z)) * sizeof(float);
   CU(cudaMemsetAsync(s->d_psi_pool, 0, psi_total, s->stream));
   CU(cudaMemsetAsync(s->d_ctr, 0, 4 * sizeof(int32_t), s->stream));
   for (int a = 0; a < 6; ++a)
@@ -1089,7 +1110,7 @@ static void release_second_buffer(sim *s) {
   dfree(s->d_psib_pool);
   s->d_psib_pool = NULL;
   s->device_bytes -= (uint64_t)6 * s->cells * sizeof(float) +
-                     (uint64_t)4 * (s->size_x + s->size_y + s->size_z) * sizeof(float);
+                     (uint64_t)(s->psi_x + s->psi_y + s->psi_z) * sizeof(float);
   s->fused = 0;
 }
 
@@ -1185,6 +1206,77 @@ static int fused_mode(void) {
   return -1;
 }
 
+/* The multi-step kernel's counters and its probe lists by z-plane. */
+static int flow_setup(sim *s) {
+  int rc;
+  const int64_t n = fdtdk_flow_counters(s->J, s->K);
+  if ((rc = dalloc(s, (void **)&s->d_flow, (size_t)n * sizeof(uint32_t)))) return rc;
+  s->flow_zeroed = 0;
+  /* Item height: a half-step should have an item or more for each of the
+   * 456 groups (3 on each of 152 SMs), then as many planes as that leaves,
+   * since an item's waits, first loads and face pass cost as much as several
+   * planes.  Measured from rest (us a step at 1/2/4/8 planes an item; mode 0,
+   * then mode 5): 64^3 11.1/14.0/21.4/- and 26.5/29.7/34.6/-; 80^3 13/16/22/36
+   * and 34/30/34/48; 112^3 30/25/28/38 and 70/54/41/49; 144^3 61/49/48/58 and
+   * 112/91/73/72; 192^3 -/102/96/97 and -/153/123/117; modes 1-4 lie between.
+   * 16 planes are slower everywhere.  Tile: 32 x 16 has the least halo; on the
+   * largest grids the longer rows of 64 x 8 read better (512x512x448: 1387
+   * against 1419; 400^3 no difference). */
+  s->flow_tile = s->cells >= ((int64_t)1 << 26) ? 0 : 1;
+  s->flow_zc = s->cells < 350000 ? 1 : s->cells < 1100000 ? 2 : s->cells < 6000000 ? 4 : 8;
+  if (s->flow_zc > s->K) s->flow_zc = s->K;
+  s->n_pat = 0;
+  if (!s->init_ant || s->num_ant <= 0) return FDTD_OK;
+  const int K = s->K;
+  int32_t *pz = (int32_t *)calloc((size_t)K + 1, sizeof(int32_t));
+  int32_t *pat = (int32_t *)calloc((size_t)s->num_ant * 4, sizeof(int32_t));
+  int32_t *at = (int32_t *)calloc((size_t)K, sizeof(int32_t));
+  if (!pz || !pat || !at) {
+    free(pz);
+    free(pat);
+    free(at);
+    return fail(FDTD_ERR_OOM, "out of host memory");
+  }
+  /* a probe belongs to the H item whose cells hold it, the last plane, row
+   * and column to the ones before them */
+  for (int pass = 0; pass < 2; ++pass) {
+    for (int a = 0; a < s->num_ant; ++a) {
+      const int64_t id = s->h_probe_idx[a];
+      if (id < 0) continue; /* outside: its record stays zero */
+      const int k = (int)(id / s->plane), j = (int)(id % s->plane / s->Ip);
+      const int i = (int)(id % s->Ip), kk = k < K - 2 ? k : K - 2;
+      if (pass == 0) {
+        pz[kk + 1] += 1;
+        /* the last row of the last plane: E there is not among what the H
+         * item waits for */
+        if (k == K - 1 && j == s->J - 1) s->n_pat = -1;
+      } else {
+        int32_t *e = pat + 4 * (size_t)(pz[kk] + at[kk]++);
+        e[0] = a;
+        e[1] = i;
+        e[2] = j;
+      }
+    }
+    if (pass == 0)
+      for (int k = 0; k < K; ++k) pz[k + 1] += pz[k];
+  }
+  const size_t zb = ((size_t)K + 1) * sizeof(int32_t), ab = (size_t)s->num_ant * 4 * sizeof(int32_t);
+  if (!(rc = dalloc(s, (void **)&s->d_pz, zb))) rc = dalloc(s, (void **)&s->d_pat, ab);
+  cudaError_t e = cudaSuccess;
+  if (!rc) {
+    e = cudaMemcpyAsync(s->d_pz, pz, zb, cudaMemcpyHostToDevice, s->stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(s->d_pat, pat, ab, cudaMemcpyHostToDevice, s->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
+    if (s->n_pat == 0) s->n_pat = s->num_ant;
+  }
+  free(pz);
+  free(pat);
+  free(at);
+  if (rc) return rc;
+  CU(e);
+  return FDTD_OK;
+}
+
 /* src/simulation.h:640-979 */
 int fdtd_ready_simulation(fdtd_handle h) {
   GET(h);
@@ -1231,8 +1323,9 @@ int fdtd_ready_simulation(fdtd_handle h) {
   }
   const size_t bytes = (size_t)s->cells * sizeof(float);
   int rc;
-  for (int a = 0; a < 6; ++a)
-    if ((rc = dalloc(s, (void **)&s->d_f[a], bytes))) return rc;
+  s->fstride = (s->cells + 63) / 64 * 64; /* 256-byte aligned fields */
+  if ((rc = dalloc(s, (void **)&s->d_f[0], 6 * (size_t)s->fstride * sizeof(float)))) return rc;
+  for (int a = 1; a < 6; ++a) s->d_f[a] = s->d_f[0] + a * s->fstride;
   if ((rc = dalloc(s, (void **)&s->d_mat, (size_t)s->cells * sizeof(uint16_t)))) return rc;
   CU(cudaMemsetAsync(s->d_mat, 0, (size_t)s->cells * sizeof(uint16_t), s->stream));
   if (s->allow_compress) {
@@ -1247,8 +1340,8 @@ int fdtd_ready_simulation(fdtd_handle h) {
   CU(cudaMemsetAsync(s->d_err, 0, sizeof(int32_t), s->stream));
   /* floats per pair array: 2 slabs of size_* cells, 2 values per cell */
   const int64_t psi_n[FDTD_NUM_PSI] = {
-      [PSI_EY] = 4 * s->size_y, [PSI_HY] = 4 * s->size_y, [PSI_EZ] = 4 * s->size_z,
-      [PSI_HZ] = 4 * s->size_z, [PSI_EX] = 4 * s->size_x, [PSI_HX] = 4 * s->size_x};
+      [PSI_EY] = s->psi_y, [PSI_HY] = s->psi_y, [PSI_EZ] = s->psi_z,
+      [PSI_HZ] = s->psi_z, [PSI_EX] = s->psi_x, [PSI_HX] = s->psi_x};
   int64_t psi_total = 0;
   for (int a = 0; a < FDTD_NUM_PSI; ++a) psi_total += psi_n[a];
   if ((rc = dalloc(s, (void **)&s->d_psi_pool, (size_t)psi_total * sizeof(float)))) return rc;
@@ -1260,6 +1353,7 @@ int fdtd_ready_simulation(fdtd_handle h) {
     }
   }
   const int fmode = fused_mode();
+  s->fused_forced = fmode == 1;
   if (s->use_tma && (fmode == 1 || (fmode < 0 && tune_enabled() &&
                                     s->cells >= TUNE_MIN_CELLS))) { /* the fused step's second buffer */
     for (int a = 0; a < 6; ++a)
@@ -1283,12 +1377,15 @@ int fdtd_ready_simulation(fdtd_handle h) {
     CU(cudaMemcpyAsync(s->d_probe_idx, s->h_probe_idx, (size_t)s->num_ant * sizeof(int64_t),
                        cudaMemcpyHostToDevice, s->stream));
   }
+  if (s->use_tma && (rc = flow_setup(s))) return rc;
   fill_dev_struct(s);
   if ((rc = upload_coefficients(s))) return rc;
   if ((rc = zero_state(s))) return rc;
   if (s->use_tma) {
     for (int t = 0; t < FDTD_NUM_TILES; ++t)
       if (fdtdk_make_maps(&s->dev, t, &s->maps[t])) s->maps[t].valid = 0;
+    for (int t = 0; t < FDTD_FLOW_TILES; ++t)
+      if (fdtdk_make_maps_flow(&s->dev, t, s->fstride, &s->wmaps[t])) s->wmaps[t].valid = 0;
     if (!s->maps[0].valid) /* the direct kernels take over */
       for (int t = 1; t < FDTD_NUM_TILES; ++t) s->maps[t].valid = 0;
   }
@@ -1326,6 +1423,31 @@ typedef struct {
   int32_t version, I, J, K, Ip, p, T, num_ant, coef_mode, pad;
   int64_t psi_floats, probe_floats;
 } ckpt_header;
+
+/* Copies the psi pairs between the device arrays' padded rows and the
+ * image's dense ones (dense: device memory, psi_floats values). */
+static int ckpt_psi(sim *s, float *dense, int to_dense) {
+  const size_t pair = 2 * sizeof(float);
+  const int p = s->p;
+  float *at = dense;
+  for (int a = 0; a < FDTD_NUM_PSI; ++a) {
+    const int x = a == PSI_EX || a == PSI_HX, y = a == PSI_EY || a == PSI_HY;
+    const size_t rows = x ? (size_t)s->J * s->K : (y ? (size_t)2 * p * s->K : (size_t)2 * p * s->J);
+    const size_t pitch = (size_t)(x ? s->pxp : s->Ip) * pair;
+    const size_t width = (size_t)(x ? 2 * p : s->I) * pair;
+    for (int part = 0; part < (x ? 2 : 1); ++part) { /* X: the low and the high slab */
+      unsigned char *pad = (unsigned char *)s->d_psi[a] + (part ? (size_t)(p + s->pxo) * pair : 0);
+      unsigned char *den = (unsigned char *)at + (part ? (size_t)p * pair : 0);
+      const size_t w = x ? (size_t)p * pair : width;
+      if (to_dense)
+        CU(cudaMemcpy2DAsync(den, width, pad, pitch, w, rows, cudaMemcpyDeviceToDevice, s->stream));
+      else
+        CU(cudaMemcpy2DAsync(pad, pitch, den, width, w, rows, cudaMemcpyDeviceToDevice, s->stream));
+    }
+    at += rows * (width / sizeof(float));
+  }
+  return FDTD_OK;
+}
 
 static void ckpt_describe(const sim *s, ckpt_header *hd) {
   memset(hd, 0, sizeof(*hd));
@@ -1374,8 +1496,15 @@ int fdtd_checkpoint_save(fdtd_handle h, void *buf, size_t n) {
   const size_t fb = (size_t)s->cells * sizeof(float);
   for (int a = 0; a < 6; ++a, o += fb)
     CU(cudaMemcpyAsync(o, s->d_f[a], fb, cudaMemcpyDeviceToHost, s->stream));
-  CU(cudaMemcpyAsync(o, s->d_psi_pool, (size_t)hd.psi_floats * sizeof(float),
-                     cudaMemcpyDeviceToHost, s->stream));
+  const size_t pb = (size_t)hd.psi_floats * sizeof(float);
+  float *dense = NULL;
+  CU(pool_alloc((void **)&dense, pb, s->stream));
+  rc = ckpt_psi(s, dense, 1);
+  const cudaError_t pe =
+      rc ? cudaSuccess : cudaMemcpyAsync(o, dense, pb, cudaMemcpyDeviceToHost, s->stream);
+  dfree(dense);
+  if (rc) return rc;
+  CU(pe);
   o += (size_t)hd.psi_floats * sizeof(float);
   CU(cudaMemcpyAsync(o, s->d_ctr, 4 * sizeof(int32_t), cudaMemcpyDeviceToHost, s->stream));
   o += 4 * sizeof(int32_t);
@@ -1406,8 +1535,14 @@ int fdtd_checkpoint_load(fdtd_handle h, const void *buf, size_t n) {
   const size_t fb = (size_t)s->cells * sizeof(float);
   for (int a = 0; a < 6; ++a, o += fb)
     CU(cudaMemcpyAsync(s->d_f[a], o, fb, cudaMemcpyHostToDevice, s->stream));
-  CU(cudaMemcpyAsync(s->d_psi_pool, o, (size_t)want.psi_floats * sizeof(float),
-                     cudaMemcpyHostToDevice, s->stream));
+  const size_t pb = (size_t)want.psi_floats * sizeof(float);
+  float *dense = NULL;
+  CU(pool_alloc((void **)&dense, pb, s->stream));
+  const cudaError_t pe = cudaMemcpyAsync(dense, o, pb, cudaMemcpyHostToDevice, s->stream);
+  rc = pe == cudaSuccess ? ckpt_psi(s, dense, 0) : FDTD_OK;
+  dfree(dense);
+  CU(pe);
+  if (rc) return rc;
   o += (size_t)want.psi_floats * sizeof(float);
   CU(cudaMemcpyAsync(s->d_ctr, o, 4 * sizeof(int32_t), cudaMemcpyHostToDevice, s->stream));
   o += 4 * sizeof(int32_t);
@@ -1745,6 +1880,7 @@ static int check_device_error(sim *s) {
   CU(cudaStreamSynchronize(s->stream));
   if (e) {
     cudaMemsetAsync(s->d_err, 0, sizeof(int32_t), s->stream);
+    s->flow_zeroed = 0; /* its row counters may have stopped anywhere */
     return fail(FDTD_ERR_CUDA, "a TMA pipeline wait timed out in a half-step kernel "
                                "(device error word %d); the fields are not valid", e);
   }
@@ -1997,24 +2133,30 @@ int fdtd_add_currents(fdtd_handle h, int32_t step, int32_t mode, const int32_t b
 
 /* ------------------------------------------------------------ fused loop */
 
-static int step_ops(sim *s, int32_t step, int from_dev, int32_t mode, const fdtd_current *cur) {
-  fdtd_op oh, oe;
-  memset(&oh, 0, sizeof(oh));
-  oh.curl = 1;
-  oh.pml = 1;
-  oh.tfsf_mode = mode;
-  oh.step = step;
-  oh.step_from_dev = from_dev;
-  oe = oh;
+/* The E half-step of a whole step: curl, CPML, TF/SF mode, current source
+ * (none when its box is empty or negative: the reference touches no cell). */
+static void step_op_e(fdtd_op *o, int32_t mode, const fdtd_current *cur) {
+  memset(o, 0, sizeof(*o));
+  o->curl = 1;
+  o->pml = 1;
+  o->tfsf_mode = mode;
   if (cur && cur->mode >= 1 && cur->mode <= 3) {
     int ok = 1;
     for (int a = 0; a < 6; ++a) ok &= cur->box[a] >= 0;
     ok &= cur->box[1] >= cur->box[0] && cur->box[3] >= cur->box[2] && cur->box[5] >= cur->box[4];
     if (ok) {
-      oe.cur_mode = cur->mode;
-      memcpy(oe.cur_box, cur->box, sizeof(oe.cur_box));
+      o->cur_mode = cur->mode;
+      memcpy(o->cur_box, cur->box, sizeof(o->cur_box));
     }
   }
+}
+
+static int step_ops(sim *s, int32_t step, int from_dev, int32_t mode, const fdtd_current *cur) {
+  fdtd_op oh, oe;
+  step_op_e(&oe, mode, cur);
+  step_op_e(&oh, mode, NULL);
+  oh.step = oe.step = step;
+  oh.step_from_dev = oe.step_from_dev = from_dev;
   if (s->dev.num_ant > 0) KL(fdtdk_probe_gather(&s->dev, s->stream));
   int rc = issue(s, 1, &oh);
   if (rc) return rc;
@@ -2115,6 +2257,64 @@ static int run_fused(sim *s, int32_t first, int32_t count, int32_t mode) {
   return FDTD_OK;
 }
 
+#define FLOW_MIN_OBLIQUE 65536 /* cells */
+
+/* Can steps of this mode (and current) run as multi-step launches? */
+static int flow_usable(sim *s, int32_t mode, const fdtd_current *cur) {
+  /* Mode 5 corrects every component on all six faces.  On a tiny grid that is
+   * most of an item's time, and separate kernels spread it better (us a step,
+   * separate / this way: 24^3 24/35, 48^3 31/26, 64^3 27/27, 96^3 50/37). */
+  if (mode == FDTD_MODE_OBLIQUE && s->cells < FLOW_MIN_OBLIQUE) return 0;
+  if (!s->use_tma || !s->maps[0].valid || !s->d_flow || s->n_pat < 0) return 0;
+  if (!s->wmaps[s->flow_tile].valid) return 0;
+  if (s->dev.num_ant > 0 && s->n_pat == 0) return 0;
+  fdtd_op o;
+  step_op_e(&o, mode, cur);
+  return fdtd_flow_ok(&s->dev, &o);
+}
+
+/* One launch of n steps from `first` with the handle's item geometry. */
+static int flow_launch(sim *s, int32_t first, int32_t n, int32_t mode, const fdtd_current *cur) {
+  fdtd_flow w;
+  memset(&w, 0, sizeof(w));
+  if (!s->flow_zeroed) {
+    CU(cudaMemsetAsync(s->d_flow, 0,
+                       (size_t)fdtdk_flow_counters(s->J, s->K) * sizeof(uint32_t), s->stream));
+    s->flow_zeroed = 1;
+    s->flow_base = 0;
+  }
+  w.n_steps = n;
+  w.first = first;
+  w.base = s->flow_base;
+  w.cnt = s->d_flow;
+  w.tile = s->flow_tile;
+  w.zc = s->flow_zc;
+  if (s->dev.num_ant > 0) {
+    w.probe_z = s->d_pz;
+    w.probe_at = s->d_pat;
+    w.n_probes = s->n_pat;
+  }
+  fdtd_op o;
+  step_op_e(&o, mode, cur);
+  KL(fdtdk_flow(&s->dev, s->wmaps, &o, &w, s->stream));
+  s->flow_base += (uint32_t)n;
+  return FDTD_OK;
+}
+
+static int run_flow(sim *s, int32_t first, int32_t count, int32_t mode, const fdtd_current *cur) {
+  /* a launch's tickets fit its 32-bit counter many times over */
+  const int64_t items = 2 * (int64_t)((s->I + 31) / 32) * ((s->J + 3) / 4) * (s->K / s->flow_zc + 1);
+  int64_t most = ((int64_t)1 << 28) / items;
+  if (most < 1) most = 1;
+  for (int32_t done = 0; done < count;) {
+    const int32_t n = count - done < most ? count - done : (int32_t)most;
+    const int rc = flow_launch(s, first + done, n, mode, cur);
+    if (rc) return rc;
+    done += n;
+  }
+  return FDTD_OK;
+}
+
 /* Steps first..first+count-1 as GRAPH_CHUNK-step graph replays and single
  * steps (the arguments already checked). */
 static int run_steps(sim *s, int32_t first, int32_t count, int32_t mode,
@@ -2123,6 +2323,10 @@ static int run_steps(sim *s, int32_t first, int32_t count, int32_t mode,
   const int use_cur = cur && cur->mode >= 1 && cur->mode <= 3;
   const int probes = s->dev.num_ant > 0;
   int32_t done = 0;
+  /* Multi-step launches unless FDTD_FUSED=1 asked for the fused pairs: they
+   * are faster than either other way at every size measured (flow_usable). */
+  const int forced = s->fused_forced && fused_usable(s, mode, cur);
+  if (!forced && flow_usable(s, mode, cur)) return run_flow(s, first, count, mode, cur);
   if (count >= 2 && fused_usable(s, mode, cur)) return run_fused(s, first, count, mode);
   if (count >= GRAPH_CHUNK) {
     const int cm = use_cur ? cur->mode : 0;
@@ -2271,16 +2475,18 @@ int fdtd_estimate_device_bytes(int32_t I, int32_t J, int32_t K, int32_t pml, int
                 pml, T);
   const uint64_t Ip = (uint64_t)(I + 7) / 8 * 8, cells = Ip * (uint64_t)J * (uint64_t)K;
   const uint64_t S = (uint64_t)(I > J ? (I > K ? I : K) : (J > K ? J : K));
-  const uint64_t sx = (uint64_t)pml * J * K, sy = (uint64_t)I * pml * K,
-                 sz = (uint64_t)I * J * pml;
-  uint64_t b = 6 * cells * 4;                      /* fields */
+  const uint64_t psi = 2 * (uint64_t)fdtd_psi_x_pitch(I, pml) * J * K + 4 * (uint64_t)pml * Ip * K +
+                       4 * (uint64_t)pml * Ip * J; /* floats of a family's three arrays */
+  uint64_t b = 6 * (cells + 63) * 4;               /* fields */
   b += 6 * cells * 4;                              /* coefficients (until indexed) */
   b += cells * 2 + (uint64_t)MAX_MATERIALS * 6 * 4; /* material ids + table */
   b += (uint64_t)HASH_CAP * (8 + 8 + 4) + 16 + 4;  /* indexing scratch, error word */
-  b += 8 * (sx + sy + sz) * 4;                     /* psi pairs */
+  b += 2 * psi * 4;                                /* psi pairs */
+  b += (uint64_t)fdtdk_flow_counters(J, K) * 4 +
+       ((uint64_t)K + 1 + 4 * (uint64_t)num_ant) * 4; /* multi-step counters, probe lists */
   if (fused_mode() == 1 || (fused_mode() < 0 && tune_enabled() &&
                               (int64_t)cells >= TUNE_MIN_CELLS))
-    b += 6 * cells * 4 + 4 * (sx + sy + sz) * 4;   /* the fused step's second buffer
+    b += 6 * cells * 4 + psi * 4;                  /* the fused step's second buffer
                                                       (held until the autotuner decides) */
   b += 2 * (uint64_t)I * 4 + 16;                   /* stretch denominators, counters */
   b += (uint64_t)T * num_ant * 6 * 4 + (uint64_t)num_ant * 8; /* probes */

@@ -26,9 +26,9 @@ extern "C" {
  * The reference keeps them as twelve separate arrays (src/simulation.h);
  * the values and their slab indexing are the same. */
 enum {
-  PSI_EY = 0, /* {psi_Exy, psi_Ezy}, index i + py*I + k*2p*I */
-  PSI_EZ,     /* {psi_Exz, psi_Eyz}, index i + j*I + pz*I*J   */
-  PSI_EX,     /* {psi_Eyx, psi_Ezx}, index px + j*2p + k*2p*J */
+  PSI_EY = 0, /* {psi_Exy, psi_Ezy}, index i + py*Ip + k*2p*Ip */
+  PSI_EZ,     /* {psi_Exz, psi_Eyz}, index i + j*Ip + pz*Ip*J   */
+  PSI_EX,     /* {psi_Eyx, psi_Ezx}, index xpos(px) + (j + k*J)*pitch */
   PSI_HY,     /* {psi_Hxy, psi_Hzy} */
   PSI_HX,     /* {psi_Hyx, psi_Hzx} */
   PSI_HZ      /* {psi_Hxz, psi_Hyz} */
@@ -38,7 +38,11 @@ enum {
  * Field, coefficient and material-id arrays are pitched: cell (i,j,k) is
  * at i + j*Ip + k*Ip*J with Ip = I rounded up to a multiple of 8, so that
  * every row starts 32-byte aligned and TMA strides are multiples of 16 B.
- * CPML psi arrays and the 1D tables keep the reference's dense layouts. */
+ * The rows of the CPML psi pairs are padded too, so that the pairs of four
+ * cells i..i+3 with i a multiple of 4 are one aligned 32-byte access on every
+ * axis: Y and Z rows have the fields' pitch; an X row holds the low slab's p
+ * positions from 0 and the high slab's further on, such that cell i and its
+ * position agree modulo 4 (fdtd_psi_x_off, fdtd_psi_x_pitch).  The 1D tables are dense. */
 typedef struct {
   int32_t I, J, K, p;
   int32_t Ip;               /* row pitch (elements) */
@@ -93,6 +97,21 @@ typedef struct {
   int32_t tile_h, tile_e;
 } fdtd_dev;
 
+/* Layout of the X psi rows for an axis of I cells (the high slab starts at
+ * cell I - p): slab position px is at px, from p on at px + off; pitch a
+ * multiple of 4. */
+#ifdef __CUDACC__
+#define FDTD_HD __host__ __device__
+#else
+#define FDTD_HD
+#endif
+FDTD_HD static inline int32_t fdtd_psi_x_off(int32_t I, int32_t p) {
+  return ((p + 3) & ~3) + ((I - p) & 3) - p;
+}
+FDTD_HD static inline int32_t fdtd_psi_x_pitch(int32_t I, int32_t p) {
+  return ((p + 3) & ~3) + ((((I - p) & 3) + p + 3) & ~3);
+}
+
 /* TMA descriptors (CUtensorMap, 128 B each) of one grid in one tile
  * geometry: 0..5 = Ex Ey Ez Hx Hy Hz as E-half-step boxes, 6..11 the same
  * arrays as H-half-step boxes, 12 = material ids.  Opaque to C.  A handle
@@ -109,6 +128,16 @@ typedef struct {
   FDTD_ALIGN64 unsigned char bytes[FDTD_NUM_MAPS][128];
   int32_t valid;            /* 1 when every map encoded */
 } fdtd_maps;
+
+/* The multi-step kernel's descriptors (fdtd_flow.cu): the three components of
+ * a family at once (the fields are one allocation, fstride values apart): E
+ * and H as tiles, E and H with the halo, the material ids. */
+#define FDTD_FLOW_MAPS 5
+#define FDTD_FLOW_TILES 2 /* tile geometries it runs in: 0, 1 */
+typedef struct {
+  FDTD_ALIGN64 unsigned char bytes[FDTD_FLOW_MAPS][128];
+  int32_t valid;
+} fdtd_maps_flow;
 
 /* One fused half-step: which parts run, for which step. */
 typedef struct {
@@ -213,6 +242,43 @@ static inline int fdtd_fused_ok(const fdtd_dev *d, const fdtd_op *op) {
   if (d->i1 > d->I - p - 3 || d->j1 > d->J - p - 3 || d->k1 > d->K - p - 3) return 0;
   return d->i0 <= d->i1 && d->j0 <= d->j1 && d->k0 <= d->k1;
 }
+
+/* Many whole steps in one launch (fdtd_flow.cu): curl, TF/SF, CPML and the
+ * current source of every cell in one pass per half-step.  Can steps of this E
+ * op (its H op is the same without the current source) run that way?  A face
+ * cell takes its TF/SF correction after the curl and the CPML there, so the
+ * faces must be clear of the CPML; the current source comes last either way,
+ * except that mode 5 with the source on a face is refused. */
+static inline int fdtd_flow_ok(const fdtd_dev *d, const fdtd_op *op) {
+  if (!op->curl || !op->pml || d->p < 1) return 0;
+  /* no four cells i..i+3 (i a multiple of 4) in both x slabs */
+  if (((d->I - d->p) & ~3) < ((d->p + 3) & ~3)) return 0;
+  { /* psi offsets in 32 bits */
+    const int64_t jk = d->J > d->K ? d->J : d->K;
+    if (2 * (int64_t)d->p * d->Ip * jk > 0x7fffffff) return 0;
+    if ((int64_t)fdtd_psi_x_pitch(d->I, d->p) * d->J * d->K > 0x7fffffff) return 0;
+  }
+  if (!op->tfsf_mode) return 1;
+  if (op->tfsf_mode == FDTD_MODE_OBLIQUE) return d->ob_inc[0] && fdtd_tfsf_faces_clear(d, op);
+  fdtd_op o = *op;
+  o.cur_mode = 0;
+  return d->inc[0] && fdtd_tfsf_faces_clear(d, &o);
+}
+typedef struct {
+  int32_t n_steps, first;   /* steps first .. first + n_steps - 1 */
+  uint32_t base;            /* steps the counters have seen since they were zeroed */
+  uint32_t *cnt;            /* fdtdk_flow_counters values */
+  int32_t tile, zc;         /* tile geometry, z-planes per item */
+  const int32_t *probe_z;   /* [K+1] first probe entry of each z-plane */
+  const int32_t *probe_at;  /* {probe, i, j, 0} by plane */
+  int32_t n_probes;
+} fdtd_flow;
+/* Counters a grid needs at any tile geometry and item height. */
+int64_t fdtdk_flow_counters(int32_t J, int32_t K);
+/* Runs the steps of op (its E half-step; step_from_dev unused) in one launch. */
+int fdtdk_make_maps_flow(const fdtd_dev *d, int tile, int64_t fstride, fdtd_maps_flow *m);
+int fdtdk_flow(const fdtd_dev *d, const fdtd_maps_flow *m, const fdtd_op *op, const fdtd_flow *w,
+               cudaStream_t s);
 
 /* Launchers (fdtd_kernels.cu).  Return cudaError_t as int.  m: the maps
  * of every tile geometry (FDTD_NUM_TILES).  With valid maps and op->curl

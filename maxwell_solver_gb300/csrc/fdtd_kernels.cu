@@ -140,7 +140,7 @@ __global__ void __launch_bounds__(TX *TY) k_half_e(const fdtd_dev d, const fdtd_
     const Coef6 C = load_coef(d, n);
     float ex = Ex[n], ey = Ey[n], ez = Ez[n];
     update_e_cell<CURL, PML>(d, mode, inc, cm, cur_src, cur, i, j, k, px, py, pz, C, ex, ey,
-                             ez, hx, hy, hz, hz_jm, hx_jm, hz_im, hy_im, hx_km, hy_km);
+                             ez, hx, hy, hz, hz_jm, hx_jm, hz_im, hy_im, hx_km, hy_km, d.bE, d.cE);
     Ex[n] = ex;
     Ey[n] = ey;
     Ez[n] = ez;
@@ -381,22 +381,6 @@ __global__ void k_init_1d_oblique(float *E, float *H, int n1, int m_src, int mb,
   }
 }
 
-// Window value at coordinate x (linear interpolation between nodes).
-__device__ __forceinline__ float ob_interp(const float *row, float x, int w) {
-  int m = (int)floorf(x);
-  m = m < 0 ? 0 : (m > w - 2 ? w - 2 : m);
-  const float f = x - (float)m;
-  return row[m] + f * (row[m + 1] - row[m]);
-}
-
-// Window coordinate of a point (px, py, pz) in cells: ob_rho 1D nodes per
-// cell of distance along k.
-__device__ __forceinline__ float ob_coord(const fdtd_dev &d, float px, float py, float pz) {
-  const float s = d.ob_k[0] * (px - (float)d.ob_r0[0]) + d.ob_k[1] * (py - (float)d.ob_r0[1]) +
-                  d.ob_k[2] * (pz - (float)d.ob_r0[2]);
-  return d.ob_x0 + d.ob_rho * s;
-}
-
 // The oblique TF/SF corrections, one face plane per blockIdx.y = q (0..11):
 // the faces normal to AXIS = q / 4, SIDE = (q / 2) % 2 (low, high), pair
 // P = q % 2 (0: E_u with H_v, 1: E_v with H_u; u, v = the axes after AXIS).
@@ -416,22 +400,6 @@ __device__ __forceinline__ float ob_coord(const fdtd_dev &d, float px, float py,
 // The plane that comes first in the order owns such an element and applies
 // all its corrections in order, so that each element has one writer and its
 // additions happen in the oracle's sequence.
-template <int A, int CE>
-__device__ __forceinline__ float ob_e_corr(const fdtd_dev &d, const float *rowH, int x0, int x1,
-                                           int x2, int side, float c, float val) {
-  constexpr int CH = 3 - A - CE;            // the H component the face pairs with E_ce
-  constexpr bool T0 = CE == (A + 1) % 3;    // pair (E_u, H_v)
-  const int lo = A == 0 ? d.i0 : (A == 1 ? d.j0 : d.k0);
-  const int hi = A == 0 ? d.i1 : (A == 1 ? d.j1 : d.k1);
-  const int xa = side ? hi : lo - 1;        // the H cell outside the face
-  const float p0 = (float)(A == 0 ? xa : x0) + (CH != 0 ? 0.5f : 0.f);
-  const float p1 = (float)(A == 1 ? xa : x1) + (CH != 1 ? 0.5f : 0.f);
-  const float p2 = (float)(A == 2 ? xa : x2) + (CH != 2 ? 0.5f : 0.f);
-  const float inc = d.ob_h[CH] * ob_interp(rowH, ob_coord(d, p0, p1, p2) - 0.5f, d.ob_w);
-  const float t = c * inc;
-  return (T0 == (side == 0)) ? val + t : val - t;
-}
-
 template <bool HFAM, int Q>
 __device__ __forceinline__ void ob_plane(const fdtd_dev &d, int step, int first, int stride) {
   constexpr int AXIS = Q >> 2, SIDE = (Q >> 1) & 1, P = Q & 1;

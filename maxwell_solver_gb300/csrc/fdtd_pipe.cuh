@@ -64,6 +64,7 @@ __device__ __forceinline__ bool mbar_wait_for(uint64_t *bar, uint32_t parity,
                                               unsigned long long limit_ns) {
   if (mbar_try_wait(bar, parity)) return true;
   const unsigned long long t0 = global_ns();
+#pragma unroll 1
   for (unsigned it = 1; it < kSpinLimit; ++it) {
     if (mbar_try_wait(bar, parity)) return true;
     if ((it & 31u) == 0u && global_ns() - t0 > limit_ns) return false;
@@ -92,6 +93,14 @@ __device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, u
       : "memory");
 }
 
+__device__ __forceinline__ void tma_load_4d(void *dst, const CUtensorMap *map, uint64_t *bar,
+                                            int x, int y, int z, int c) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(smem_u32(dst)),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(c), "r"(smem_u32(bar))
+      : "memory");
+}
 
 // ------------------------------------------------------------------ host
 
@@ -122,5 +131,21 @@ inline int encode(CUtensorMap *out, void *base, CUtensorMapDataType dt, int esiz
   return r == CUDA_SUCCESS ? 0 : (int)cudaErrorInvalidValue;
 }
 
+// Three field arrays `stride` elements apart as one 4-D map: a box holds the
+// three components' tiles one after the other.
+inline int encode3(CUtensorMap *out, void *base, const fdtd_dev *d, int64_t stride, int boxw,
+                   int boxh) {
+  PFN_cuTensorMapEncodeTiled_v12000 enc = encoder();
+  if (!enc) return (int)cudaErrorNotSupported;
+  const cuuint64_t gdim[4] = {(cuuint64_t)d->I, (cuuint64_t)d->J, (cuuint64_t)d->K, 3};
+  const cuuint64_t gstride[3] = {(cuuint64_t)d->Ip * 4, (cuuint64_t)d->plane * 4,
+                                 (cuuint64_t)stride * 4};
+  const cuuint32_t box[4] = {(cuuint32_t)boxw, (cuuint32_t)boxh, 1, 3};
+  const cuuint32_t estr[4] = {1, 1, 1, 1};
+  CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, base, gdim, gstride, box, estr,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : (int)cudaErrorInvalidValue;
+}
 
 }  // namespace fdtd_pipe

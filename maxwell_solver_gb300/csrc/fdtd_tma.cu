@@ -46,16 +46,16 @@
 #include "fdtd_device.cuh"
 #include "fdtd_internal.h"
 #include "fdtd_pipe.cuh"
+#include "fdtd_tile.cuh"
 
 using namespace fdtd;
 using namespace fdtd_pipe;
+using namespace fdtd_tile;
 
 extern "C" void fdtdk_count_launches(unsigned long long n);
 
 namespace {
 
-constexpr int NCW = 8;                       // consumer warps
-constexpr int NT = (NCW + 1) * 32;           // + one producer warp
 #ifndef FDTD_NSE
 #define FDTD_NSE 4
 #endif
@@ -90,52 +90,8 @@ constexpr int kBatchMinBlocks = FDTD_BATCH_MIN_BLOCKS;  // E (and the default fo
 constexpr int kBatchNS = FDTD_BATCH_NS;
 constexpr int kBatchMinBlocksH = FDTD_BATCH_MIN_BLOCKS_H;
 constexpr int kBatchNSH = FDTD_BATCH_NS_H;
-// Tile geometry: a work item is a BX x BY tile of cells over a run of
-// z-planes.  The single-grid kernels use 64 x 8; the batched ones 32 x 16,
-// since their grids are narrow (32..128 cells in x) and a 64-wide tile of a
-// 70-cell axis leaves most lanes of its second tile idle.  Both have the
-// same stage byte sizes.
-template <int BX_, int BY_>
-struct Geo {
-  static constexpr int BX = BX_, BY = BY_;
-  static constexpr int HW = BX + 4;                   // halo box row (floats)
-  static constexpr int HH = BY + 1;                   // halo box rows
-  static constexpr int TILE_B = BX * BY * 4;          // 2048 B
-  static constexpr int HALO_B = HW * HH * 4;          // bytes transferred
-  static constexpr int HALO_SLOT = (HALO_B + 127) / 128 * 128;  // 128-byte aligned slot
-  static constexpr int MAT_B = BX * BY * 2;           // 1024 B
-  static constexpr int E_OFF_H = 3 * TILE_B;
-  static constexpr int E_OFF_M = E_OFF_H + 3 * HALO_SLOT;
-  static constexpr int E_STAGE = E_OFF_M + MAT_B;
-  static constexpr int H_OFF_H = 3 * HALO_SLOT;
-  static constexpr int H_STAGE = H_OFF_H + 3 * TILE_B;
-  static_assert(BX % 32 == 0 && (256 / 32) % (BX / 32) == 0 && BX * BY == 512,
-                "8 consumer warps, two cells per thread");
-  static_assert(E_STAGE % 128 == 0 && H_STAGE % 128 == 0, "stage alignment");
-  static_assert((HW * 4) % 16 == 0 && (BX * 4) % 16 == 0 && (BX * 2) % 16 == 0,
-                "TMA inner box extents must be multiples of 16 bytes");
-};
-using GS = Geo<64, 8>;   // single-grid kernels (tile 0, the default)
-using GB = Geo<32, 16>;  // batched kernels; single-grid tile 1 (narrow grids)
-using GW = Geo<128, 4>;  // single-grid tile 2 (wide grids)
 template <bool BATCH>
 using GeoOf = typename std::conditional<BATCH, GB, GS>::type;
-// The single-grid tile geometry by index (fdtd_dev::tile_e / tile_h).
-template <int T>
-using TileGeo = typename std::conditional<T == 0, GS,
-                                          typename std::conditional<T == 1, GB, GW>::type>::type;
-constexpr int kSmemTabMax = 512;             // coefficient ids staged in shared memory
-constexpr int CTRL_B = 512;                  // barriers + stage metadata
-// Batch mode: every stage also carries its grid's descriptor and op (bulk
-// copies completing on the stage's barrier), so the per-cell code reads
-// them from shared memory instead of global memory; E stages also carry
-// the grid's coefficient table when it has at most kStageTabMax ids.
-constexpr int DESC_B = 1536;                 // >= sizeof(fdtd_dev), 128-aligned
-constexpr int OPSLOT_B = 128;                // >= sizeof(fdtd_op)
-constexpr int kStageTabMax = 64;
-constexpr int TAB_B = kStageTabMax * 6 * 4;  // 1536 B
-static_assert(sizeof(fdtd_dev) <= DESC_B && sizeof(fdtd_dev) % 16 == 0, "descriptor slot");
-static_assert(sizeof(fdtd_op) <= OPSLOT_B && sizeof(fdtd_op) % 16 == 0, "op slot");
 template <bool BATCH, class G = GeoOf<BATCH>>
 struct EG {
   static constexpr int NS = BATCH ? kBatchNS : NSE;
@@ -160,10 +116,6 @@ static_assert(kBatchMinBlocks * (EG<true>::SMEM + 1024) <= 228 * 1024 &&
 static_assert(NSH * (8 + 8 + 32) <= CTRL_B && NSE * (8 + 8 + 32) <= CTRL_B &&
                   kBatchNS * (8 + 8 + 32) <= CTRL_B && kBatchNSH * (8 + 8 + 32) <= CTRL_B,
               "control block");
-
-struct Maps {
-  CUtensorMap m[FDTD_NUM_MAPS];
-};
 
 // Work items of one launch.  Single grid: a regular decomposition of the
 // grid (tiles_x * tiles_y tiles x z-runs of zchunk planes).  Batch: an
@@ -272,18 +224,6 @@ __device__ void produce(const Items &it, int extra, uint64_t *full, uint64_t *em
   if (!ok && it.err) atomicExch(it.err, 3);
   // drain: every copy issued by this block has landed before it retires
   for (int r = (q > NS ? q - NS : 0); r < q; ++r) mbar_wait(&full[r % NS], (uint32_t)((r / NS) & 1));
-}
-
-// Thread -> cell map of the consumer warps: warp w covers one 32-cell x run
-// (run w % (BX/32) of the tile's row) of rows r0 = w / (BX/32) and
-// r0 + BY/2, so that whole warps fall inside or outside the CPML x slabs and
-// TF/SF x faces.
-template <class G>
-__device__ __forceinline__ void cell_map(int tid, int &xo, int &r0) {
-  constexpr int WPR = G::BX / 32;  // warps per tile row
-  const int w = tid >> 5;
-  xo = 32 * (w % WPR) + (tid & 31);
-  r0 = w / WPR;
 }
 
 // The CPML X columns of a warp's 32-cell run as at most two runs of lanes
@@ -508,7 +448,7 @@ __global__ void __launch_bounds__(NT, BATCH ? kBatchMinBlocks : FDTD_MIN_BLOCKS_
           const bool cur = cur_col[c] && in_range(k, op.cur_box[4], op.cur_box[5]);
           update_e_cell<true, PML>(d, mode, inc, cm, cur_src, cur, i, j, k, px, py, pz, C, ex,
                                    ey, ez, hx, hy, hz, hz_jm, hx_jm, hz_im, hy_im, hx_km[c],
-                                   hy_km[c]);
+                                   hy_km[c], d.bE, d.cE);
         }
       } else {  // interior warp: i, j, k >= 1, no CPML, TF/SF face or source
         ex = C.exe * ex + C.exh * (+(hz - hz_jm) - (hy - hy_km[c]));
