@@ -39,8 +39,12 @@
  *
  * Measured (us a step, separate kernels / this): 64^3 mode 3 27.7/14.4;
  * 131x117x109 mode 5 64.8/56.4; 176x160x129 mode 4 with coefficient arrays
- * 120/80; 256^3 mode 5 281/231; 400x360x120 with a current 314/240;
- * 512x512x448 mode 1 1492/1387.
+ * 120/80; 256^3 mode 5 281/220; 400x360x120 with a current 314/226;
+ * 512x512x448 mode 1 1492/1354.  From 256^3 on that is 80-90 % of the measured
+ * copy bandwidth for two passes over the fields a step (74 B a cell and the
+ * pairs); running the E items a few chunks behind the H items of the same step,
+ * to find their operands in L2, waited longer than it saved (512x512x448: 1452
+ * at best against 1400).
  *
  * Results.  Every cell goes through the same per-cell arithmetic in the same
  * order as in the half-step kernels, so the fields, psi pairs and probe
@@ -270,6 +274,10 @@ __device__ __forceinline__ P4 ldp4(const float2 *p) {
                : "l"(p)
                : "memory");
   return r;
+}
+// Starts bringing a line to L2.
+__device__ __forceinline__ void to_l2(const void *p) {
+  asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
 }
 __device__ __forceinline__ void stp4(float2 *p, const P4 &r) {
   asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p),
@@ -631,7 +639,9 @@ __device__ __noinline__ void gather_probes(const fdtd_dev &d, const int32_t *pz,
 // MU: per-cell H coefficients (fdtd_set_magnetic; more registers, two groups).
 // OB: mode 5.  TAB: material ids with a table that fits shared memory.  One
 // kernel each, since what a step does not need would cost it instruction cache.
-template <int NG, bool MU, bool OB, bool TAB, class G>
+// AHEAD: the pairs of the next plane are brought to L2 a plane ahead, for grids
+// that do not stay there (fdtd_flow::ahead).
+template <int NG, bool MU, bool OB, bool TAB, bool AHEAD, class G>
 __global__ void __launch_bounds__(kThreads<NG>, 1)
     k_flow(const __grid_constant__ fdtd_dev d, const __grid_constant__ fdtd_op op,
            const __grid_constant__ FlowMaps mp, const __grid_constant__ Flow f) {
@@ -848,6 +858,13 @@ __global__ void __launch_bounds__(kThreads<NG>, 1)
         else if (sx) ps = ldp4(psi_pairs(d, PSI_HX) + ox);
         else if (nv > 0 && pz >= 0) ps = ldp4(psi_pairs(d, PSI_HZ) + (oz + (int64_t)pz * d.plane));
       };
+      // The next plane's pairs are on their way to L2 meanwhile.
+      const auto ahead = [&](int k, int y, int x) {
+        const int pz = slab_h(k, K, p);
+        if (sy) to_l2(psi_pairs(d, PSI_HY) + y);
+        if (sx) to_l2(psi_pairs(d, PSI_HX) + x);
+        if (nv > 0 && pz >= 0) to_l2(psi_pairs(d, PSI_HZ) + (oz + (int64_t)pz * d.plane));
+      };
       // An item with nothing but the curl for this warp (all its cells H cells
       // outside the CPML) has a loop of its own: about 110 instructions a plane
       // against 300 and a call, and no path test.
@@ -901,6 +918,7 @@ __global__ void __launch_bounds__(kThreads<NG>, 1)
             // CPML Y, X, Z (gpu.h:644-685, :604-642, :687-725)
             const int pz = slab_h(k, K, p);
             const bool sz = nv > 0 && pz >= 0;
+            if (AHEAD && k > kb) ahead(k - 1, oy - sY, ox - sX);
             if (nv < 4) {  // cells past the last H cell: no recurrence
               const Q4 none = all4(0.f);
               const uint32_t past = 0xfu << max(nv, 0);
@@ -991,6 +1009,12 @@ __global__ void __launch_bounds__(kThreads<NG>, 1)
           ps = ldp4(psi_pairs(d, PSI_EZ) + (oz + (int64_t)pz * d.plane));
         else if (sx_ && k_in) ps = ldp4(psi_pairs(d, PSI_EX) + ox);
       };
+      const auto ahead = [&](int k, int y, int x) {
+        const int pz = slab_e(k, K, p);
+        if (py >= 0) to_l2(psi_pairs(d, PSI_EY) + y);
+        if (sx_) to_l2(psi_pairs(d, PSI_EX) + x);
+        if (nv > 0 && pz >= 0) to_l2(psi_pairs(d, PSI_EZ) + (oz + (int64_t)pz * d.plane));
+      };
       const auto planes = [&](auto curl_only) {
         constexpr bool kCurl = decltype(curl_only)::value;
         if constexpr (!kCurl) first_pairs(kb);
@@ -1069,6 +1093,7 @@ __global__ void __launch_bounds__(kThreads<NG>, 1)
             const bool k_in = k >= 1 && k <= K - 2;
             const int pz = slab_e(k, K, p);
             const bool sy = py >= 0 && k_in, sz = nv > 0 && pz >= 0 && j_in, sx = sx_ && k_in;
+            if (AHEAD && k + 1 < kb + np) ahead(k + 1, oy + sY, ox + sX);
             if (i == 0 || i + 3 > I - 2) {  // Y, Z: 1 <= i <= I-2
               const Q4 none = all4(0.f);
               const uint32_t off = (i == 0 ? 1u : 0u) | 0xfu << min(max(I - 1 - i, 0), 4);
@@ -1178,14 +1203,14 @@ int prepare(K kern, int threads, int smem, int *cached) {
   return 0;
 }
 
-template <bool MU, bool OB, bool TAB, class G>
+template <bool MU, bool OB, bool TAB, bool AHEAD, class G>
 int launch(const fdtd_dev *d, const fdtd_maps_flow *m, const fdtd_op *op, const fdtd_flow *w,
            cudaStream_t s) {
   static_assert(sizeof(FlowMaps) == sizeof(((fdtd_maps_flow *)0)->bytes), "map layout");
   static int cached = 0;
   constexpr int NG = kGroups<MU>;
   constexpr int smem = FG<NG, G>::SMEM;
-  auto kern = k_flow<NG, MU, OB, TAB, G>;
+  auto kern = k_flow<NG, MU, OB, TAB, AHEAD, G>;
   if (const int e = prepare(kern, kThreads<NG>, smem, &cached)) return e;
   FlowMaps mp;
   memcpy(&mp, m->bytes, sizeof(FlowMaps));
@@ -1225,8 +1250,9 @@ int launch(const fdtd_dev *d, const fdtd_maps_flow *m, const fdtd_op *op, const 
 template <bool MU, bool OB, bool TAB>
 int launch_tiled(const fdtd_dev *d, const fdtd_maps_flow *m, const fdtd_op *op, const fdtd_flow *w,
                  cudaStream_t s) {
-  return w->tile == 0 ? launch<MU, OB, TAB, GS>(d, &m[0], op, w, s)
-                      : launch<MU, OB, TAB, GB>(d, &m[1], op, w, s);
+  if (w->tile == 0) return launch<MU, OB, TAB, true, GS>(d, &m[0], op, w, s);
+  return w->ahead ? launch<MU, OB, TAB, true, GB>(d, &m[1], op, w, s)
+                  : launch<MU, OB, TAB, false, GB>(d, &m[1], op, w, s);
 }
 template <bool MU, bool OB>
 int launch_coef(const fdtd_dev *d, const fdtd_maps_flow *m, const fdtd_op *op, const fdtd_flow *w,

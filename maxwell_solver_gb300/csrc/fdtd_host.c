@@ -1207,7 +1207,9 @@ static int fused_mode(void) {
   return -1;
 }
 
-/* The multi-step kernel's counters and its probe lists by z-plane. */
+/* The multi-step kernel's counters, its item geometry and its probe lists by
+ * z-plane. */
+#define FLOW_BIG 4000000 /* cells */
 static int flow_setup(sim *s) {
   int rc;
   const int64_t n = fdtdk_flow_counters(s->J, s->K);
@@ -1220,11 +1222,19 @@ static int flow_setup(sim *s) {
    * then mode 5): 64^3 11.1/14.0/21.4/- and 26.5/29.7/34.6/-; 80^3 13/16/22/36
    * and 34/30/34/48; 112^3 30/25/28/38 and 70/54/41/49; 144^3 61/49/48/58 and
    * 112/91/73/72; 192^3 -/102/96/97 and -/153/123/117; modes 1-4 lie between.
-   * 16 planes are slower everywhere.  Tile: 32 x 16 has the least halo; on the
-   * largest grids the longer rows of 64 x 8 read better (512x512x448: 1387
-   * against 1419; 400^3 no difference). */
-  s->flow_tile = s->cells >= ((int64_t)1 << 26) ? 0 : 1;
-  s->flow_zc = s->cells < 350000 ? 1 : s->cells < 1100000 ? 2 : s->cells < 6000000 ? 4 : 8;
+   * 16 planes are slower everywhere.
+   *
+   * From 4 million cells on the fields (24 B a cell) and the psi pairs outgrow
+   * the L2 cache, and the pairs are fetched ahead (without / with, 8 planes:
+   * 128^3 54/55 in mode 5, 160^3 80/74, 256^3 238/225, 320^3 439/418).
+   *
+   * Tile: 32 x 16 has the least halo and fits narrow grids; the longer rows of
+   * 64 x 8 read better from memory (32 x 16 / 64 x 8, mode 1, 8 planes: 240^3
+   * 182/189, 288^3 292/304, 320^3 396/389, 448^3 1068/1019, 1200x100x100
+   * 168/159, 512x512x448 1381/1354). */
+  const int big = s->cells >= FLOW_BIG;
+  s->flow_tile = big && s->I >= 320 ? 0 : 1;
+  s->flow_zc = s->cells < 350000 ? 1 : s->cells < 1100000 ? 2 : big ? 8 : 4;
   if (s->flow_zc > s->K) s->flow_zc = s->K;
   s->n_pat = 0;
   if (!s->init_ant || s->num_ant <= 0) return FDTD_OK;
@@ -2298,6 +2308,7 @@ static int flow_launch(sim *s, int32_t first, int32_t n, int32_t mode, const fdt
   w.cnt = s->d_flow;
   w.tile = s->flow_tile;
   w.zc = s->flow_zc;
+  w.ahead = s->cells >= FLOW_BIG;
   if (s->dev.num_ant > 0) {
     w.probe_z = s->d_pz;
     w.probe_at = s->d_pat;

@@ -1,6 +1,6 @@
 """Steps as multi-step launches (fdtd_flow.cu) against the FP32 oracle, bit
 for bit (every route does the same roundings, so the tolerance is zero): each
-item height (1, 2, 4 and 8 planes, by grid size) with partial tiles, partial
+item height (1, 2, 4 and 8 planes, by grid size) and tile with partial tiles, partial
 chunks and rows that are not a multiple of four cells, TF/SF modes, current
 sources, coefficient arrays, per-cell H coefficients, and probes on the last
 planes.  A run is split into several calls, so that launches go on from each
@@ -28,7 +28,9 @@ CASES = {
     "oblique_four_planes": ((130, 117, 109), 9, 11, 60, 5, ""),
     "two_planes": ((97, 81, 67), 10, 12, 48, 3, "current"),
     "four_planes": ((129, 95, 78), 9, 11, 48, 2, "magnetic"),
-    "eight_planes": ((198, 145, 131), 10, 12, 48, 1, ""),
+    "big": ((198, 155, 131), 10, 12, 48, 1, ""),
+    "big_oblique": ((165, 173, 142), 9, 11, 64, 5, "magnetic"),
+    "big_wide": ((331, 113, 109), 8, 10, 48, 3, "current arrays"),
 }
 
 
