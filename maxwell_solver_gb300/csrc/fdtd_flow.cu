@@ -1221,7 +1221,7 @@ int launch(const fdtd_dev *d, const fdtd_maps_flow *m, const fdtd_op *op, const 
   f.base = w->base;
   f.work = d->work;
   f.cnt = w->cnt;
-  f.err = d->err;
+  f.err = w->err;
   f.zc = w->zc;
   f.nch_h = (d->K - 1 + w->zc - 1) / w->zc;
   f.nch_e = (d->K + w->zc - 1) / w->zc;
@@ -1241,7 +1241,8 @@ int launch(const fdtd_dev *d, const fdtd_maps_flow *m, const fdtd_op *op, const 
   f.probe_at = reinterpret_cast<const int4 *>(w->probe_at);
   f.n_probes = w->n_probes;
   const long long want = (2ll * f.tiles * f.nch_e + NG - 1) / NG;  // a step's items
-  const int blocks = want < cached ? (int)want : cached;
+  int blocks = want < cached ? (int)want : cached;
+  if (w->blocks > 0 && w->blocks < blocks) blocks = w->blocks;
   kern<<<blocks, kThreads<NG>, smem, s>>>(*d, *op, mp, f);
   fdtdk_count_launches(1);
   return (int)cudaGetLastError();

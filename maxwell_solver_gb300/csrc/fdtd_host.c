@@ -169,11 +169,11 @@ typedef struct sim {
   int gf_mode, gf_probes;
   unsigned long long gf_kernels;
   /* many steps per launch (fdtd_flow.cu): the row counters, the steps they
-   * have counted since they were zeroed, the probes by z-plane, and the item
-   * geometry */
+   * have counted since they were zeroed and the item height they were zeroed
+   * for (0: not zeroed), the item geometry, and the probes by z-plane */
   uint32_t *d_flow;
   uint32_t flow_base;
-  int flow_zeroed;
+  int32_t flow_counted;
   int32_t flow_tile, flow_zc;
   int32_t *d_pz, *d_pat, n_pat;     /* n_pat -1: a probe position it cannot serve */
 } sim;
@@ -1214,7 +1214,7 @@ static int flow_setup(sim *s) {
   int rc;
   const int64_t n = fdtdk_flow_counters(s->J, s->K);
   if ((rc = dalloc(s, (void **)&s->d_flow, (size_t)n * sizeof(uint32_t)))) return rc;
-  s->flow_zeroed = 0;
+  s->flow_counted = 0;
   /* Item height: a half-step should have an item or more for each of the
    * 456 groups (3 on each of 152 SMs), then as many planes as that leaves,
    * since an item's waits, first loads and face pass cost as much as several
@@ -1891,7 +1891,7 @@ static int check_device_error(sim *s) {
   CU(cudaStreamSynchronize(s->stream));
   if (e) {
     cudaMemsetAsync(s->d_err, 0, sizeof(int32_t), s->stream);
-    s->flow_zeroed = 0; /* its row counters may have stopped anywhere */
+    s->flow_counted = 0; /* its row counters may have stopped anywhere */
     return fail(FDTD_ERR_CUDA, "a TMA pipeline wait timed out in a half-step kernel "
                                "(device error word %d); the fields are not valid", e);
   }
@@ -2276,14 +2276,8 @@ static int run_fused(sim *s, int32_t first, int32_t count, int32_t mode) {
   return FDTD_OK;
 }
 
-#define FLOW_MIN_OBLIQUE 65536 /* cells */
-
 /* Can steps of this mode (and current) run as multi-step launches? */
-static int flow_usable(sim *s, int32_t mode, const fdtd_current *cur) {
-  /* Mode 5 corrects every component on all six faces.  On a tiny grid that is
-   * most of an item's time, and separate kernels spread it better (us a step,
-   * separate / this way: 24^3 24/35, 48^3 31/26, 64^3 27/27, 96^3 50/37). */
-  if (mode == FDTD_MODE_OBLIQUE && s->cells < FLOW_MIN_OBLIQUE) return 0;
+static int flow_possible(sim *s, int32_t mode, const fdtd_current *cur) {
   if (!s->use_tma || !s->maps[0].valid || !s->d_flow || s->n_pat < 0) return 0;
   if (!s->wmaps[s->flow_tile].valid) return 0;
   if (s->dev.num_ant > 0 && s->n_pat == 0) return 0;
@@ -2292,23 +2286,32 @@ static int flow_usable(sim *s, int32_t mode, const fdtd_current *cur) {
   return fdtd_flow_ok(&s->dev, &o);
 }
 
-/* One launch of n steps from `first` with the handle's item geometry. */
-static int flow_launch(sim *s, int32_t first, int32_t n, int32_t mode, const fdtd_current *cur) {
+/* Mode 5 corrects every component on all six faces.  On a tiny grid of its own
+ * that is most of an item's time, and separate kernels spread it better (us a
+ * step, separate / this way: 24^3 24/35, 48^3 31/26, 64^3 27/27, 96^3 50/37). */
+#define FLOW_MIN_OBLIQUE 65536 /* cells */
+static int flow_usable(sim *s, int32_t mode, const fdtd_current *cur) {
+  return (mode != FDTD_MODE_OBLIQUE || s->cells >= FLOW_MIN_OBLIQUE) && flow_possible(s, mode, cur);
+}
+
+/* n steps from `first` on the handle's stream, zc planes an item; on at most
+ * `blocks` SMs (0: all), errors reported in *err (device). */
+static int run_flow(sim *s, int32_t first, int32_t count, int32_t mode, const fdtd_current *cur,
+                    int32_t zc, int32_t blocks, int32_t *err) {
   fdtd_flow w;
   memset(&w, 0, sizeof(w));
-  if (!s->flow_zeroed) {
+  if (s->flow_counted != zc) {
     CU(cudaMemsetAsync(s->d_flow, 0,
                        (size_t)fdtdk_flow_counters(s->J, s->K) * sizeof(uint32_t), s->stream));
-    s->flow_zeroed = 1;
+    s->flow_counted = zc;
     s->flow_base = 0;
   }
-  w.n_steps = n;
-  w.first = first;
-  w.base = s->flow_base;
   w.cnt = s->d_flow;
   w.tile = s->flow_tile;
-  w.zc = s->flow_zc;
+  w.zc = zc;
   w.ahead = s->cells >= FLOW_BIG;
+  w.blocks = blocks;
+  w.err = err;
   if (s->dev.num_ant > 0) {
     w.probe_z = s->d_pz;
     w.probe_at = s->d_pat;
@@ -2316,21 +2319,16 @@ static int flow_launch(sim *s, int32_t first, int32_t n, int32_t mode, const fdt
   }
   fdtd_op o;
   step_op_e(&o, mode, cur);
-  KL(fdtdk_flow(&s->dev, s->wmaps, &o, &w, s->stream));
-  s->flow_base += (uint32_t)n;
-  return FDTD_OK;
-}
-
-static int run_flow(sim *s, int32_t first, int32_t count, int32_t mode, const fdtd_current *cur) {
-  /* a launch's tickets fit its 32-bit counter many times over */
-  const int64_t items = 2 * (int64_t)((s->I + 31) / 32) * ((s->J + 3) / 4) * (s->K / s->flow_zc + 1);
-  int64_t most = ((int64_t)1 << 28) / items;
-  if (most < 1) most = 1;
-  for (int32_t done = 0; done < count;) {
-    const int32_t n = count - done < most ? count - done : (int32_t)most;
-    const int rc = flow_launch(s, first + done, n, mode, cur);
-    if (rc) return rc;
-    done += n;
+  /* A launch lasts some 10 ms at most, so that other streams' work gets its
+   * turn; its tickets then fit their 32-bit counter many times over. */
+  const int64_t cs = (int64_t)1 << (blocks ? 31 : 29);
+  const int32_t most = s->cells < cs / 8 ? (int32_t)(cs / s->cells) : 8;
+  for (int32_t done = 0; done < count; done += w.n_steps) {
+    w.n_steps = count - done < most ? count - done : most;
+    w.first = first + done;
+    w.base = s->flow_base;
+    KL(fdtdk_flow(&s->dev, s->wmaps, &o, &w, s->stream));
+    s->flow_base += (uint32_t)w.n_steps;
   }
   return FDTD_OK;
 }
@@ -2346,7 +2344,8 @@ static int run_steps(sim *s, int32_t first, int32_t count, int32_t mode,
   /* Multi-step launches unless FDTD_FUSED=1 asked for the fused pairs: they
    * are faster than either other way at every size measured (flow_usable). */
   const int forced = s->fused_forced && fused_usable(s, mode, cur);
-  if (!forced && flow_usable(s, mode, cur)) return run_flow(s, first, count, mode, cur);
+  if (!forced && flow_usable(s, mode, cur))
+    return run_flow(s, first, count, mode, cur, s->flow_zc, 0, s->d_err);
   if (count >= 2 && fused_usable(s, mode, cur)) return run_fused(s, first, count, mode);
   if (count >= GRAPH_CHUNK) {
     const int cm = use_cur ? cur->mode : 0;
@@ -2760,12 +2759,14 @@ int fdtd_create_signal(double fctr, double delT, double percentage_bw, double nu
 
 /* ==================================================================== batch
  *
- * A batch advances many simulation handles of different sizes together:
- * every batched step is one H and one E launch of the persistent TMA kernels
- * over the work items of all active members (plus a probe gather and a step
- * counter update), so small grids fill the GPU together instead of each
- * leaving most of it idle.  The per-cell arithmetic is the single-grid
- * kernels', so every member ends bit-identical to running it alone.
+ * A batch advances many simulation handles of different sizes together, so
+ * that small grids fill the GPU together instead of each leaving most of it
+ * idle.  When the members are few and their steps can run as multi-step launches,
+ * each gets its share of the SMs and runs there on its own stream (batch_flow).
+ * Otherwise every batched step is one H and one E launch of the persistent TMA
+ * kernels over the work items of all active members (plus a probe gather and a
+ * step counter update).  The per-cell arithmetic is the single-grid kernels',
+ * so every member ends bit-identical to running it alone.
  */
 
 #define MAX_BATCHES 256
@@ -2808,7 +2809,7 @@ typedef struct batch {
   unsigned char *d_maps;
   fdtd_op *d_ops;
   int32_t *d_steps, *d_tab_h, *d_tab_e, *d_work, *d_err;
-  int dev_cap, cap_h, cap_e;
+  int dev_cap, cap_h, cap_e, act_cap;
   /* host staging */
   fdtd_dev *h_devs;
   unsigned char *h_maps;
@@ -2816,6 +2817,9 @@ typedef struct batch {
   int32_t *h_steps, *h_tab_h, *h_tab_e;
   int *act;  /* member index of each active slot */
   int n_act, n_h, n_e, any_probes, dirty;
+  int flow;        /* the active members run as multi-step launches */
+  int mirrored;    /* the device mirrors hold the active set */
+  int own_work;    /* b->stream has work on members' fields */
   int any_split;   /* some active member's TF/SF runs as the face pass */
   int any_oblique; /* ... in mode 5 */
   int32_t face_max; /* largest face-plane area of those members */
@@ -2861,6 +2865,7 @@ int fdtd_batch_create(fdtd_batch *out) {
   if (e == cudaSuccess) e = pool_alloc((void **)&b->d_err, sizeof(int32_t), b->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(b->d_work, 0, 4 * sizeof(int32_t), b->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(b->d_err, 0, sizeof(int32_t), b->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream); /* d_err: on the members' streams */
   if (e != cudaSuccess) {
     free(b);
     return fail(FDTD_ERR_CUDA, "batch create: %s", cudaGetErrorString(e));
@@ -2911,7 +2916,7 @@ static void batch_free_mirrors(batch *b) {
   b->h_ops = NULL;
   b->h_steps = b->h_tab_h = b->h_tab_e = NULL;
   b->act = NULL;
-  b->dev_cap = b->cap_h = b->cap_e = 0;
+  b->dev_cap = b->cap_h = b->cap_e = b->act_cap = 0;
 }
 
 int fdtd_batch_destroy(fdtd_batch h) {
@@ -3073,9 +3078,6 @@ static int batch_rebuild_(batch *b) {
     b->d_maps = NULL;
     b->d_ops = NULL;
     b->d_steps = NULL;
-    free(b->act);
-    b->act = (int *)malloc((size_t)cap * sizeof(int));
-    if (!b->act) return fail(FDTD_ERR_OOM, "out of host memory");
     if ((rc = ensure_cap((void **)&b->d_devs, (void **)&b->h_devs, &c0, cap, sizeof(fdtd_dev),
                          b->stream)))
       return rc;
@@ -3111,7 +3113,6 @@ static int batch_rebuild_(batch *b) {
     const bmember *m = &b->m[i];
     if (m->done >= m->count) continue;
     sim *s = lookup(m->h);
-    b->act[g] = i;
     b->h_devs[g] = s->dev;
     memcpy(b->h_maps + (size_t)g * mapsz, s->maps[1].bytes, mapsz);
     fdtd_op *op = &b->h_ops[g];
@@ -3148,7 +3149,6 @@ static int batch_rebuild_(batch *b) {
     ne = add_items(b->h_tab_e, ne, g, s->I, s->J, s->K, b->zrun);
     ++g;
   }
-  b->n_act = na;
   b->n_h = nh;
   b->n_e = ne;
   if (na) {
@@ -3167,8 +3167,125 @@ static int batch_rebuild_(batch *b) {
     /* the staging buffers are reused by the next rebuild: wait for the copies */
     CU(cudaStreamSynchronize(b->stream));
   }
+  b->mirrored = 1;
+  return FDTD_OK;
+}
+
+static int sm_count(void) {
+  int sms = 0, dev = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms < 1 ? 1 : sms;
+}
+
+/* The active members, and how they run. */
+static int batch_list(batch *b) {
+  if (b->n > b->act_cap) {
+    int *a = (int *)realloc(b->act, (size_t)b->n * sizeof(int));
+    if (!a) return fail(FDTD_ERR_OOM, "out of host memory");
+    b->act = a;
+    b->act_cap = b->n;
+  }
+  b->n_act = 0;
+  for (int i = 0; i < b->n; ++i) {
+    const bmember *m = &b->m[i];
+    if (m->done >= m->count) continue;
+    sim *s = lookup(m->h);
+    if (!s) return fail(FDTD_ERR_INVALID_HANDLE, "a batch member was deleted");
+    b->act[b->n_act++] = i;
+  }
+  /* On their own SMs the members need several each: with fewer, rounding the
+   * shares to whole SMs and the rate of one SM on a small grid cost more than
+   * the launches.  300 steps of members of 32..128 cells a side, mode 5, separate
+   * kernels / multi-step launches (ms): 4 members 29.6/18.4, 8 48.7/40.3, 16
+   * 53.3/42.6, 20 73.2/62.2, 24 94.0/97.0, 32 104/109; 600 steps of 48 293/357.
+   * 100..200 cells, mode 1, 100 steps: 4 39.2/23.0, 16 86.1/74.0. */
+  b->flow = b->n_act * 7 <= sm_count();
+  for (int g = 0; g < b->n_act && b->flow; ++g) {
+    const bmember *m = &b->m[b->act[g]];
+    b->flow = flow_possible(lookup(m->h), m->mode, m->has_cur ? &m->cur : NULL);
+  }
+  b->mirrored = 0;
   b->dirty = 0;
   return FDTD_OK;
+}
+
+/* The active members' streams (or, with to_batch, the batch's stream after
+ * them) wait for the batch's work so far. */
+static int batch_order(batch *b, int to_batch) {
+  if (!to_batch) CU(cudaEventRecord(b->ev, b->stream));
+  for (int g = 0; g < b->n_act; ++g) {
+    sim *s = lookup(b->m[b->act[g]].h);
+    if (!s) return fail(FDTD_ERR_INVALID_HANDLE, "a batch member was deleted");
+    if (to_batch) {
+      CU(cudaEventRecord(s->ev[15], s->stream));
+      CU(cudaStreamWaitEvent(b->stream, s->ev[15], 0));
+    } else {
+      CU(cudaStreamWaitEvent(s->stream, b->ev, 0));
+    }
+  }
+  return FDTD_OK;
+}
+
+/* A member's share of a multi-step round: its work and its SMs. */
+typedef struct {
+  int g;          /* active slot */
+  double work;
+  int32_t blocks;
+} bshare;
+static int by_work(const void *x, const void *y) {
+  const double a = ((const bshare *)x)->work, b = ((const bshare *)y)->work;
+  return a < b ? 1 : (a > b ? -1 : 0);
+}
+
+/* The active members' next steps (steps[g] of each) as multi-step launches,
+ * every member on its own stream and its own SMs, the longest first.  Shares:
+ * the smallest time t for which ceil(work / t) SMs for every member with more
+ * than t of work, and work / t for the others (which follow each other on the
+ * SMs that become free), are no more than the GPU has.  A cell in the CPML
+ * counts for three (160^3 and 400^3 differ by 1.22 in their rate, 1.29 by this
+ * weight).  Members wait for nothing of each other. */
+static int batch_flow(batch *b, const int32_t *steps) {
+  const int sms = sm_count();
+  bshare *sh = (bshare *)malloc((size_t)b->n_act * sizeof(bshare));
+  if (!sh) return fail(FDTD_ERR_OOM, "out of host memory");
+  double lo = 0, hi = 0;
+  for (int g = 0; g < b->n_act; ++g) {
+    const sim *s = lookup(b->m[b->act[g]].h);
+    if (!s) {
+      free(sh);
+      return fail(FDTD_ERR_INVALID_HANDLE, "a batch member was deleted");
+    }
+    const double in = (double)(s->I - 2 * s->p) * (s->J - 2 * s->p) * (s->K - 2 * s->p);
+    sh[g].g = g;
+    sh[g].work = (3.0 * s->cells - 2.0 * (in > 0 ? in : 0)) * steps[g];
+    hi += sh[g].work;
+  }
+  qsort(sh, (size_t)b->n_act, sizeof(*sh), by_work);
+  for (int it = 0; it < 40; ++it) { /* hi: enough for one SM */
+    const double t = 0.5 * (lo + hi);
+    double need = 0;
+    for (int g = 0; g < b->n_act; ++g) need += sh[g].work > t ? ceil(sh[g].work / t) : sh[g].work / t;
+    if (need <= sms) hi = t;
+    else lo = t;
+  }
+  int rc = FDTD_OK;
+  for (int g = 0; g < b->n_act && !rc; ++g) {
+    const bmember *m = &b->m[b->act[sh[g].g]];
+    sim *s = lookup(m->h);
+    const double share = ceil(sh[g].work / hi);
+    const int32_t blocks = share < 1 ? 1 : (share > sms ? sms : (int32_t)share);
+    /* items as in flow_setup's rule, for this member's part of the SMs */
+    const double at_all = (double)s->cells * sms / blocks;
+    int32_t zc = at_all < 350000 ? 1 : at_all < 1100000 ? 2 : at_all < FLOW_BIG ? 4 : 8;
+    if (zc > s->K) zc = s->K;
+    rc = run_flow(s, m->first + m->done, steps[sh[g].g], m->mode, m->has_cur ? &m->cur : NULL, zc,
+                  blocks, b->d_err);
+  }
+  free(sh);
+  /* the batch's stream follows every member: after all launches, since the
+   * streams share a few hardware queues and a wait holds its queue up */
+  return rc ? rc : batch_order(b, 1);
 }
 
 /* One step of every active member: the probe rows, H (+ faces), E (+ x-slab
@@ -3249,32 +3366,25 @@ int fdtd_batch_get_zrun(fdtd_batch bh, int32_t *zrun) {
   return FDTD_OK;
 }
 
-/* Advances every active member by up to max_steps steps (all by the same
- * number: the fewest remaining steps of any active member, capped by
- * max_steps).  *active_left receives the number of members still running. */
-int fdtd_batch_step(fdtd_batch bh, int32_t max_steps, int32_t *active_left) {
-  batch *b = blookup(bh);
-  if (!b) return fail(FDTD_ERR_INVALID_HANDLE, "invalid batch handle");
+/* Advances the active members by up to max_steps steps: all by the same number
+ * (the fewest remaining steps of any), or with to_end each by what it has left
+ * where the members run on their own. */
+static int batch_advance(batch *b, int32_t max_steps, int to_end, int32_t *active_left) {
   int rc;
   int32_t left = 0;
   for (int i = 0; i < b->n; ++i) left += b->m[i].done < b->m[i].count;
   if (active_left) *active_left = left;
   if (!left || max_steps <= 0) return FDTD_OK;
   if (b->dirty) {
+    if ((rc = batch_list(b))) return rc;
     /* new members: their own queued work must be on the device first */
-    for (int i = 0; i < b->n; ++i) {
-      if (b->m[i].done >= b->m[i].count) continue;
-      sim *s = lookup(b->m[i].h);
-      if (!s) return fail(FDTD_ERR_INVALID_HANDLE, "a batch member was deleted");
-      if ((rc = flush(s))) return rc;
-      CU(cudaEventRecord(s->ev[15], s->stream));
-      CU(cudaStreamWaitEvent(b->stream, s->ev[15], 0));
-    }
+    for (int g = 0; g < b->n_act; ++g)
+      if ((rc = flush(lookup(b->m[b->act[g]].h)))) return rc;
+    if ((rc = batch_order(b, 1))) return rc;
     if (b->gexec) { /* the mirrors and item tables change */
       cudaGraphExecDestroy(b->gexec);
       b->gexec = NULL;
     }
-    if ((rc = batch_rebuild(b))) return rc;
   }
   int32_t nsteps = max_steps;
   for (int g = 0; g < b->n_act; ++g) {
@@ -3282,61 +3392,95 @@ int fdtd_batch_step(fdtd_batch bh, int32_t max_steps, int32_t *active_left) {
     if (m->count - m->done < nsteps) nsteps = m->count - m->done;
   }
   int32_t tuned = 0; /* steps the tuning took (already counted per member) */
-  if (!b->tuned && b->n_act >= BATCH_TUNE_MIN_MEMBERS && nsteps > 4 * BATCH_TUNE_CANDS) {
-    if ((rc = batch_tune(b, &tuned))) return rc;
+  const int tune = !b->tuned && b->n_act >= BATCH_TUNE_MIN_MEMBERS && nsteps > 4 * BATCH_TUNE_CANDS;
+  if (!b->flow || tune) {
+    b->own_work = 1;
+    if (!b->mirrored && (rc = batch_rebuild(b))) return rc;
   }
-  int32_t t = tuned;
-  if (nsteps - t >= GRAPH_CHUNK) {
-    if (!b->gexec) {
-      cudaGraph_t g;
-      const double tc0 = mono_s();
-      const unsigned long long before = fdtdk_launch_count();
-      CU(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
-      int crc = FDTD_OK;
-      for (int c = 0; c < GRAPH_CHUNK && !crc; ++c) crc = batch_step_ops(b);
-      cudaError_t ce = cudaStreamEndCapture(b->stream, &g);
-      if (crc) return crc;
-      if (ce != cudaSuccess) return fail(FDTD_ERR_CUDA, "graph capture: %s", cudaGetErrorString(ce));
-      ce = cudaGraphInstantiate(&b->gexec, g, 0);
-      cudaGraphDestroy(g);
-      if (ce != cudaSuccess) {
-        b->gexec = NULL;
-        return fail(FDTD_ERR_CUDA, "graph instantiate: %s", cudaGetErrorString(ce));
+  if (tune && (rc = batch_tune(b, &tuned))) return rc;
+  if (b->flow) {
+    if (b->own_work && (rc = batch_order(b, 0))) return rc;
+    b->own_work = 0;
+    int32_t *n = (int32_t *)malloc((size_t)b->n_act * sizeof(int32_t));
+    if (!n) return fail(FDTD_ERR_OOM, "out of host memory");
+    for (int g = 0; g < b->n_act; ++g) {
+      const bmember *m = &b->m[b->act[g]];
+      const int32_t rest = m->count - m->done;
+      n[g] = !to_end ? nsteps - tuned : (rest < max_steps ? rest : max_steps);
+    }
+    rc = batch_flow(b, n);
+    for (int g = 0; g < b->n_act && !rc; ++g) {
+      bmember *m = &b->m[b->act[g]];
+      m->done += n[g];
+      if (m->done >= m->count) b->dirty = 1;
+    }
+    free(n);
+    if (rc) return rc;
+    b->mirrored = 0; /* the members' steps */
+  } else {
+    int32_t t = tuned;
+    if (nsteps - t >= GRAPH_CHUNK) {
+      if (!b->gexec) {
+        cudaGraph_t g;
+        const double tc0 = mono_s();
+        const unsigned long long before = fdtdk_launch_count();
+        CU(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
+        int crc = FDTD_OK;
+        for (int c = 0; c < GRAPH_CHUNK && !crc; ++c) crc = batch_step_ops(b);
+        cudaError_t ce = cudaStreamEndCapture(b->stream, &g);
+        if (crc) return crc;
+        if (ce != cudaSuccess)
+          return fail(FDTD_ERR_CUDA, "graph capture: %s", cudaGetErrorString(ce));
+        ce = cudaGraphInstantiate(&b->gexec, g, 0);
+        cudaGraphDestroy(g);
+        if (ce != cudaSuccess) {
+          b->gexec = NULL;
+          return fail(FDTD_ERR_CUDA, "graph instantiate: %s", cudaGetErrorString(ce));
+        }
+        b->g_kernels = fdtdk_launch_count() - before;
+        g_captured_kernels += b->g_kernels;
+        b->t_capture += mono_s() - tc0;
+        b->n_capture += 1;
       }
-      b->g_kernels = fdtdk_launch_count() - before;
-      g_captured_kernels += b->g_kernels;
-      b->t_capture += mono_s() - tc0;
-      b->n_capture += 1;
+      while (nsteps - t >= GRAPH_CHUNK) {
+        t += GRAPH_CHUNK;
+        CU(cudaGraphLaunch(b->gexec, b->stream));
+        g_graph_kernels += b->g_kernels;
+      }
     }
-    while (nsteps - t >= GRAPH_CHUNK) {
-      t += GRAPH_CHUNK;
-      CU(cudaGraphLaunch(b->gexec, b->stream));
-      g_graph_kernels += b->g_kernels;
-    }
-  }
-  for (; t < nsteps; ++t)
-    if ((rc = batch_step_ops(b))) return rc;
-  int finished = 0;
-  for (int g = 0; g < b->n_act; ++g) {
-    bmember *m = &b->m[b->act[g]];
-    m->done += nsteps - tuned;
-    if (m->done >= m->count) finished = 1;
-  }
-  if (finished) {
-    /* finished members: later calls on their handles follow the batch */
-    CU(cudaEventRecord(b->ev, b->stream));
+    for (; t < nsteps; ++t)
+      if ((rc = batch_step_ops(b))) return rc;
+    int finished = 0;
     for (int g = 0; g < b->n_act; ++g) {
       bmember *m = &b->m[b->act[g]];
-      if (m->done < m->count) continue;
-      sim *s = lookup(m->h);
-      if (s) CU(cudaStreamWaitEvent(s->stream, b->ev, 0));
+      m->done += nsteps - tuned;
+      if (m->done >= m->count) finished = 1;
     }
-    b->dirty = 1;
+    if (finished) {
+      /* finished members: later calls on their handles follow the batch */
+      CU(cudaEventRecord(b->ev, b->stream));
+      for (int g = 0; g < b->n_act; ++g) {
+        bmember *m = &b->m[b->act[g]];
+        if (m->done < m->count) continue;
+        sim *s = lookup(m->h);
+        if (s) CU(cudaStreamWaitEvent(s->stream, b->ev, 0));
+      }
+      b->dirty = 1;
+    }
   }
   left = 0;
   for (int i = 0; i < b->n; ++i) left += b->m[i].done < b->m[i].count;
   if (active_left) *active_left = left;
   return FDTD_OK;
+}
+
+/* Advances every active member by up to max_steps steps (all by the same
+ * number: the fewest remaining steps of any active member, capped by
+ * max_steps).  *active_left receives the number of members still running. */
+int fdtd_batch_step(fdtd_batch bh, int32_t max_steps, int32_t *active_left) {
+  batch *b = blookup(bh);
+  if (!b) return fail(FDTD_ERR_INVALID_HANDLE, "invalid batch handle");
+  return batch_advance(b, max_steps, 0, active_left);
 }
 
 int fdtd_internal_batch_counts(fdtd_batch bh, uint64_t n[2], double t[2]) {
@@ -3364,6 +3508,10 @@ int fdtd_batch_status(fdtd_batch bh) {
   CU(cudaMemcpy(&e, b->d_err, sizeof(e), cudaMemcpyDeviceToHost));
   if (e) {
     cudaMemset(b->d_err, 0, sizeof(int32_t));
+    for (int i = 0; i < b->n; ++i) { /* their row counters may have stopped anywhere */
+      sim *s = lookup(b->m[i].h);
+      if (s) s->flow_counted = 0;
+    }
     return fail(FDTD_ERR_CUDA, "a TMA pipeline wait timed out in a batched half-step "
                                "(device error word %d); member fields are not valid", e);
   }
@@ -3374,7 +3522,9 @@ int fdtd_batch_status(fdtd_batch bh) {
 int fdtd_batch_run(fdtd_batch bh) {
   int32_t left = 1;
   while (left) {
-    int rc = fdtd_batch_step(bh, 1 << 30, &left);
+    batch *b = blookup(bh);
+    if (!b) return fail(FDTD_ERR_INVALID_HANDLE, "invalid batch handle");
+    int rc = batch_advance(b, 1 << 30, 1, &left);
     if (rc) return rc;
   }
   return fdtd_batch_status(bh);

@@ -269,6 +269,8 @@ typedef struct {
   uint32_t base;            /* steps the counters have seen since they were zeroed */
   uint32_t *cnt;            /* fdtdk_flow_counters values */
   int32_t tile, zc;         /* tile geometry, z-planes per item */
+  int32_t blocks;           /* SMs to use at most (0: all) */
+  int32_t *err;             /* device error word */
   int32_t ahead;            /* tile 1: psi pairs come to L2 a plane ahead (tile 0: always) */
   const int32_t *probe_z;   /* [K+1] first probe entry of each z-plane */
   const int32_t *probe_at;  /* {probe, i, j, 0} by plane */

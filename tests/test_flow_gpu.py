@@ -104,3 +104,41 @@ def test_multi_step_launches_equal_oracle(name, monkeypatch):
     np.testing.assert_array_equal(rec, o.array("probes"))
     assert max(np.abs(o.field(f)).max() for f in FIELDS) > 0
     simFDTD("DeleteSimulation", P)
+
+
+def test_batch_changing_route_equals_alone():
+    """24 members run as batched half-steps; as members finish, the 21 and fewer
+    left go on as multi-step launches; a member added then starts there."""
+    from maxwell_solver_gb300 import simFDTD
+    from maxwell_solver_gb300.batch import Batch
+    from scenarios import SCENARIOS, run_mex
+
+    def ready(sc):
+        return run_mex(simFDTD, type(sc)(**{**sc.__dict__, "steps": 0}), sc.inputs())
+
+    def fields(P, sc):
+        n = np.uint32(np.prod(sc.dims))
+        return [simFDTD("OutputVis", P, n, np.int32(f)) for f in range(1, 7)]
+
+    def current(sc):
+        return (sc.cur_mode, sc.cur_box) if sc.cur_mode else None
+
+    mix = [SCENARIOS[g % len(SCENARIOS)] for g in range(25)]
+    steps = [20 + g for g in range(25)]
+    members = [ready(sc) for sc in mix]
+    with Batch() as b:
+        for P, sc, n in zip(members[:24], mix, steps):
+            b.add(P, 0, n, sc.mode, current(sc))
+        for _ in range(5):  # to the end of the first members, and past it
+            b.step(1 << 20)
+        b.add(members[24], 0, steps[24], mix[24].mode, current(mix[24]))
+        b.step(3)
+        b.run()
+        for P, sc, n in zip(members, mix, steps):
+            Q = ready(sc)
+            cur = [np.int32([sc.cur_mode, *sc.cur_box])] if sc.cur_mode else []
+            simFDTD("StepN", Q, np.int32([0, n, sc.mode]), *cur)
+            for a, w, f in zip(fields(P, sc), fields(Q, sc), FIELDS):
+                np.testing.assert_array_equal(a, w, err_msg=f"{sc.name} {n} {f}")
+            simFDTD("DeleteSimulation", Q)
+            simFDTD("DeleteSimulation", P)
