@@ -562,6 +562,7 @@ __device__ __forceinline__ void release_items(Ctrl *ctrl, uint32_t *cnt, const i
   Ctrl &c = ctrl[live ? lane : 0];
   int item = 0;
   unsigned long long t0 = global_ns();
+#pragma unroll 1
   for (unsigned it = 1; __any_sync(0xffffffffu, live); ++it) {
     const int slot = item % ND;
     const bool ready = live && mbar_test(&c.done[slot], (uint32_t)((item / ND) & 1));
@@ -655,6 +656,7 @@ __global__ void __launch_bounds__(kThreads<NG>, 1)
   // the CPML grading, indexed per lane: a shared-memory copy (the
   // by-value descriptor's would be divergent constant-bank loads)
   __shared__ float s_bc[4][2 * FDTD_MAX_PML];  // bH cH bE cE
+#pragma unroll 1
   for (int t = threadIdx.x; t < 2 * FDTD_MAX_PML; t += kThreads<NG>) {
     s_bc[0][t] = d.bH[t];
     s_bc[1][t] = d.cH[t];
@@ -663,10 +665,12 @@ __global__ void __launch_bounds__(kThreads<NG>, 1)
   }
   if (threadIdx.x < NG) {
     Ctrl &c = ctrl[threadIdx.x];
+#pragma unroll 1
     for (int s = 0; s < NS; ++s) {
       mbar_init(&c.full[s], 1);
       mbar_init(&c.empty[s], CW);
     }
+#pragma unroll 1
     for (int s = 0; s < ND; ++s) {
       mbar_init(&c.done[s], CW);
       mbar_init(&c.freed[s], 1);
@@ -675,6 +679,7 @@ __global__ void __launch_bounds__(kThreads<NG>, 1)
     mbar_init_fence();
   }
   if (TAB)
+#pragma unroll 1
     for (int t = threadIdx.x; t < d.n_mat * 6; t += kThreads<NG>)
       stab[t / 6 * kTabRow + t % 6] = __ldg(d.mat_tab + t);
   __syncthreads();
@@ -789,6 +794,7 @@ __global__ void __launch_bounds__(kThreads<NG>, 1)
       }
       if (!ok && f.err) atomicExch(f.err, 3);
       // drain: every copy issued by this block has landed before it retires
+#pragma unroll 1
       for (int r = (q > NS ? q - NS : 0); r < q; ++r)
         wait_on(&full[r % NS], (uint32_t)((r / NS) & 1));
     }
@@ -826,7 +832,7 @@ __global__ void __launch_bounds__(kThreads<NG>, 1)
     const float *tc = s_bc[m.x ? 3 : 1];
     // the thread's psi pairs, as 32-bit offsets (fdtd_flow_ok): Y and X of its
     // first plane with their plane strides, Z of slab position 0
-    const int oz = i + j * d.Ip;
+    const int oz = i + j * d.Ip, plane = (int)d.plane;
     const int sY = 2 * p * d.Ip, sX = fdtd_psi_x_pitch(I, p) * J;
     bool good;
     if (m.x == 0) {
@@ -838,8 +844,8 @@ __global__ void __launch_bounds__(kThreads<NG>, 1)
       const int k1 = kb + np - 1;
       int oy = i + (py + k1 * 2 * p) * d.Ip;
       int ox = psi_x4(I, p, i) + (j + k1 * J) * fdtd_psi_x_pitch(I, p);
-      int64_t n = i + (int64_t)j * d.Ip + (int64_t)k1 * d.plane;
-      const int64_t n_in = nv > 0 ? n : 0;  // a cell of the arrays for every lane
+      int n = oz + k1 * plane;
+      const int n_in = nv > 0 ? n : 0;  // a cell of the arrays for every lane
       Q4 ex1, ey1;
       {
         const float *sE = reinterpret_cast<const float *>(smem + s * ST) + ry * G::HW + xo;
@@ -854,16 +860,16 @@ __global__ void __launch_bounds__(kThreads<NG>, 1)
       P4 ps;
       const auto first_pairs = [&](int k) {
         const int pz = slab_h(k, K, p);
-        if (sy) ps = ldp4(psi_pairs(d, PSI_HY) + oy);
-        else if (sx) ps = ldp4(psi_pairs(d, PSI_HX) + ox);
-        else if (nv > 0 && pz >= 0) ps = ldp4(psi_pairs(d, PSI_HZ) + (oz + (int64_t)pz * d.plane));
+        const float2 *at = sy ? psi_pairs(d, PSI_HY) + oy : psi_pairs(d, PSI_HX) + ox;
+        if (!sy && !sx) at = psi_pairs(d, PSI_HZ) + (oz + pz * plane);
+        if (sy || sx || (nv > 0 && pz >= 0)) ps = ldp4(at);
       };
       // The next plane's pairs are on their way to L2 meanwhile.
       const auto ahead = [&](int k, int y, int x) {
         const int pz = slab_h(k, K, p);
         if (sy) to_l2(psi_pairs(d, PSI_HY) + y);
         if (sx) to_l2(psi_pairs(d, PSI_HX) + x);
-        if (nv > 0 && pz >= 0) to_l2(psi_pairs(d, PSI_HZ) + (oz + (int64_t)pz * d.plane));
+        if (nv > 0 && pz >= 0) to_l2(psi_pairs(d, PSI_HZ) + (oz + pz * plane));
       };
       // An item with nothing but the curl for this warp (all its cells H cells
       // outside the CPML) has a loop of its own: about 110 instructions a plane
@@ -949,7 +955,7 @@ __global__ void __launch_bounds__(kThreads<NG>, 1)
               stp4(psi_pairs(d, PSI_HX) + ox, ps);
             }
             if (sz) {
-              float2 *Z = psi_pairs(d, PSI_HZ) + (oz + (int64_t)pz * d.plane);
+              float2 *Z = psi_pairs(d, PSI_HZ) + (oz + pz * plane);
               if (sy || sx) ps = ldp4(Z);
               ps = recur(d, ps, all4(tb[pz]), all4(tc[pz]), dEy_z, dEx_z);
               corr4<true, 0>(hx, Cx, ps, dx);
@@ -968,7 +974,7 @@ __global__ void __launch_bounds__(kThreads<NG>, 1)
             stg4(d.f[4] + n, hy);
             stg4(d.f[5] + n, hz);
           }
-          n -= d.plane;
+          n -= plane;
           if constexpr (!kCurl) {
             oy -= sY;
             ox -= sX;
@@ -993,27 +999,27 @@ __global__ void __launch_bounds__(kThreads<NG>, 1)
       const bool use_mat = TAB || d.coef_mode == 1;
       int oy = i + (py + kb * 2 * p) * d.Ip;
       int ox = psi_x4(I, p, i) + (j + kb * J) * fdtd_psi_x_pitch(I, p);
-      int64_t n = i + (int64_t)j * d.Ip + (int64_t)kb * d.plane;
+      int n = oz + kb * plane;
       Q4 hx_km = all4(0.f), hy_km = hx_km;
       if (kb > 0 && nv > 0) {
-        hx_km = q4(__ldcg(reinterpret_cast<const float4 *>(d.f[3] + (n - d.plane))));
-        hy_km = q4(__ldcg(reinterpret_cast<const float4 *>(d.f[4] + (n - d.plane))));
+        hx_km = q4(__ldcg(reinterpret_cast<const float4 *>(d.f[3] + (n - plane))));
+        hy_km = q4(__ldcg(reinterpret_cast<const float4 *>(d.f[4] + (n - plane))));
       }
       // The first axis's pairs and the loop for the curl alone, as for H.
       P4 ps;
       const auto first_pairs = [&](int k) {
         const int pz = slab_e(k, K, p);
         const bool k_in = k >= 1 && k <= K - 2;
-        if (py >= 0 && k_in) ps = ldp4(psi_pairs(d, PSI_EY) + oy);
-        else if (nv > 0 && j_in && pz >= 0)
-          ps = ldp4(psi_pairs(d, PSI_EZ) + (oz + (int64_t)pz * d.plane));
-        else if (sx_ && k_in) ps = ldp4(psi_pairs(d, PSI_EX) + ox);
+        const bool y = py >= 0 && k_in, z = nv > 0 && j_in && pz >= 0, x = sx_ && k_in;
+        const float2 *at = y ? psi_pairs(d, PSI_EY) + oy : psi_pairs(d, PSI_EX) + ox;
+        if (!y && z) at = psi_pairs(d, PSI_EZ) + (oz + pz * plane);
+        if (y || z || x) ps = ldp4(at);
       };
       const auto ahead = [&](int k, int y, int x) {
         const int pz = slab_e(k, K, p);
         if (py >= 0) to_l2(psi_pairs(d, PSI_EY) + y);
         if (sx_) to_l2(psi_pairs(d, PSI_EX) + x);
-        if (nv > 0 && pz >= 0) to_l2(psi_pairs(d, PSI_EZ) + (oz + (int64_t)pz * d.plane));
+        if (nv > 0 && pz >= 0) to_l2(psi_pairs(d, PSI_EZ) + (oz + pz * plane));
       };
       const auto planes = [&](auto curl_only) {
         constexpr bool kCurl = decltype(curl_only)::value;
@@ -1059,7 +1065,7 @@ __global__ void __launch_bounds__(kThreads<NG>, 1)
               }
             }
           } else {
-            const int64_t nc = kCurl || nv > 0 ? n : 0;
+            const int nc = kCurl || nv > 0 ? n : 0;
             Ax = q4(__ldg(reinterpret_cast<const float4 *>(d.ce[0] + nc)));
             Ay = q4(__ldg(reinterpret_cast<const float4 *>(d.ce[1] + nc)));
             Az = q4(__ldg(reinterpret_cast<const float4 *>(d.ce[2] + nc)));
@@ -1109,7 +1115,7 @@ __global__ void __launch_bounds__(kThreads<NG>, 1)
               stp4(psi_pairs(d, PSI_EY) + oy, ps);
             }
             if (sz) {
-              float2 *Z = psi_pairs(d, PSI_EZ) + (oz + (int64_t)pz * d.plane);
+              float2 *Z = psi_pairs(d, PSI_EZ) + (oz + pz * plane);
               if (sy) ps = ldp4(Z);
               ps = recur(d, ps, all4(tb[pz]), all4(tc[pz]), dHy_z, dHx_z);
               corr4<false, 0>(ex, Cx, ps, dx);
@@ -1141,7 +1147,7 @@ __global__ void __launch_bounds__(kThreads<NG>, 1)
             stg4(d.f[1] + n, ey);
             stg4(d.f[2] + n, ez);
           }
-          n += d.plane;
+          n += plane;
           if constexpr (!kCurl) {
             oy += sY;
             ox += sX;

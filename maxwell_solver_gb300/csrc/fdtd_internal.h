@@ -253,6 +253,7 @@ static inline int fdtd_flow_ok(const fdtd_dev *d, const fdtd_op *op) {
   if (!op->curl || !op->pml || d->p < 1) return 0;
   /* no four cells i..i+3 (i a multiple of 4) in both x slabs */
   if (((d->I - d->p) & ~3) < ((d->p + 3) & ~3)) return 0;
+  if (d->plane * (int64_t)d->K > 0x7fffffff) return 0; /* cell offsets in 32 bits */
   { /* psi offsets in 32 bits */
     const int64_t jk = d->J > d->K ? d->J : d->K;
     if (2 * (int64_t)d->p * d->Ip * jk > 0x7fffffff) return 0;
