@@ -35,11 +35,12 @@
  * CPML axis, a face pass in batches of cells and psi loads a whole plane ahead
  * each took fewer cycles a plane and were 5-30 % slower as a whole, while one
  * kernel per mode family and coefficient layout (75-82 KB instead of 91) gained
- * 10 % at 256^3 with an oblique wave.
+ * 10 % at 256^3 with an oblique wave, and rolled set-up loops, one psi load for
+ * three axes and 32-bit cell offsets (75 to 71 KB) 8 % from 96^3 to 192^3.
  *
- * Measured (us a step, separate kernels / this): 64^3 mode 3 27.7/14.4;
- * 131x117x109 mode 5 64.8/56.4; 176x160x129 mode 4 with coefficient arrays
- * 120/80; 256^3 mode 5 281/220; 400x360x120 with a current 314/226;
+ * Measured (us a step, separate kernels / this): 64^3 mode 3 27.7/14.3;
+ * 131x117x109 mode 5 64.8/53.7; 176x160x129 mode 4 with coefficient arrays
+ * 120/76; 256^3 mode 5 281/220; 400x360x120 with a current 314/226;
  * 512x512x448 mode 1 1492/1354.  From 256^3 on that is 80-90 % of the measured
  * copy bandwidth for two passes over the fields a step (74 B a cell and the
  * pairs); running the E items a few chunks behind the H items of the same step,
@@ -82,8 +83,11 @@ namespace {
 constexpr int CW = 4;  // consumer warps of a group: 128 threads x 4 cells = a tile
 constexpr int NS = 4;  // ring stages of a group
 constexpr int ND = 4;  // items of a group between their first load and their release
-template <bool MU>
-constexpr int kGroups = MU ? 2 : 3;
+// Per-cell H coefficients take more registers: two groups of 168 each a thread
+// where the fields fit L2, three of 128 where memory latency is what a step
+// waits for (two / three, mode 1: 96^3 23/25 us, 320^3 527/462).
+template <bool MU, bool AHEAD>
+constexpr int kGroups = MU && !AHEAD ? 2 : 3;
 template <int NG>
 constexpr int kThreads = (NG * (CW + 1) + 1) * 32;
 struct Ctrl {
@@ -370,6 +374,39 @@ __device__ __forceinline__ void put_back(Q4 &to, const Q4 &from, uint32_t mask) 
     if (mask >> e & 1) set(to, e, get(from, e));
 }
 
+// The H coefficients of four cells from n (a multiple of 4; rows are padded, and
+// the ids and arrays there belong to the allocation): ids in one load and three
+// per table row, or one load per array (cell by cell it was seven loads each:
+// 160x144x130 63 us a step, now 60).
+struct H4 {
+  Q4 a[3], c[3];  // Chh.., Che..
+};
+__device__ __forceinline__ H4 hcoef4(const fdtd_dev &d, int n) {
+  H4 h;
+  if (d.hcoef_mode == 2) {
+    const ushort4 id = __ldg(reinterpret_cast<const ushort4 *>(d.hmat + n));
+    const int ids[4] = {id.x, id.y, id.z, id.w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float2 *r = reinterpret_cast<const float2 *>(d.hmat_tab + ids[e] * 6);
+      const float2 r0 = __ldg(r), r1 = __ldg(r + 1), r2 = __ldg(r + 2);
+      set(h.a[0], e, r0.x);
+      set(h.a[1], e, r0.y);
+      set(h.a[2], e, r1.x);
+      set(h.c[0], e, r1.y);
+      set(h.c[1], e, r2.x);
+      set(h.c[2], e, r2.y);
+    }
+  } else {
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      h.a[a] = q4(__ldg(reinterpret_cast<const float4 *>(d.hc + a * d.cells + n)));
+      h.c[a] = q4(__ldg(reinterpret_cast<const float4 *>(d.hc + (3 + a) * d.cells + n)));
+    }
+  }
+  return h;
+}
+
 // f +- (C * psi) * dx with the pairs' first (N = 0) or second element.
 template <bool PLUS, int N>
 __device__ __forceinline__ void corr4(Q4 &f, const Q4 &C, const P4 &ps, float dx) {
@@ -637,7 +674,7 @@ __device__ __noinline__ void gather_probes(const fdtd_dev &d, const int32_t *pz,
   }
 }
 
-// MU: per-cell H coefficients (fdtd_set_magnetic; more registers, two groups).
+// MU: per-cell H coefficients (fdtd_set_magnetic).
 // OB: mode 5.  TAB: material ids with a table that fits shared memory.  One
 // kernel each, since what a step does not need would cost it instruction cache.
 // AHEAD: the pairs of the next plane are brought to L2 a plane ahead, for grids
@@ -845,7 +882,6 @@ __global__ void __launch_bounds__(kThreads<NG>, 1)
       int oy = i + (py + k1 * 2 * p) * d.Ip;
       int ox = psi_x4(I, p, i) + (j + k1 * J) * fdtd_psi_x_pitch(I, p);
       int n = oz + k1 * plane;
-      const int n_in = nv > 0 ? n : 0;  // a cell of the arrays for every lane
       Q4 ex1, ey1;
       {
         const float *sE = reinterpret_cast<const float *>(smem + s * ST) + ry * G::HW + xo;
@@ -898,17 +934,11 @@ __global__ void __launch_bounds__(kThreads<NG>, 1)
           Q4 hx = lds4(sH), hy = lds4(sH + 512), hz = lds4(sH + 1024);
           Q4 Cx = Che, Cy = Che, Cz = Che;
           if (MU) {
-            Q4 Ax, Ay, Az;
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-              const HCoef hc = hcoef_at(d, kCurl || c < nv ? n + c : n_in);
-              set(Ax, c, hc.hhx);
-              set(Ay, c, hc.hhy);
-              set(Az, c, hc.hhz);
-              set(Cx, c, hc.hex);
-              set(Cy, c, hc.hey);
-              set(Cz, c, hc.hez);
-            }
+            const H4 hc = hcoef4(d, kCurl || nv > 0 ? n : 0);
+            const Q4 Ax = hc.a[0], Ay = hc.a[1], Az = hc.a[2];
+            Cx = hc.c[0];
+            Cy = hc.c[1];
+            Cz = hc.c[2];
             hx = mul4(Ax, hx);
             hy = mul4(Ay, hy);
             hz = mul4(Az, hz);
@@ -1214,7 +1244,7 @@ int launch(const fdtd_dev *d, const fdtd_maps_flow *m, const fdtd_op *op, const 
            cudaStream_t s) {
   static_assert(sizeof(FlowMaps) == sizeof(((fdtd_maps_flow *)0)->bytes), "map layout");
   static int cached = 0;
-  constexpr int NG = kGroups<MU>;
+  constexpr int NG = kGroups<MU, AHEAD>;
   constexpr int smem = FG<NG, G>::SMEM;
   auto kern = k_flow<NG, MU, OB, TAB, AHEAD, G>;
   if (const int e = prepare(kern, kThreads<NG>, smem, &cached)) return e;
