@@ -310,6 +310,22 @@ __device__ __noinline__ float2 quot_pair(float2 a, float2 q, float dx, float y) 
   return make_float2(quot_small(a.x, q.x, dx, y), quot_small(a.y, q.y, dx, y));
 }
 
+// All eight quotients of a recurrence in one call.
+struct F8 {
+  float2 v[4];
+};
+__device__ __noinline__ F8 quot_all(F8 a, F8 q, float dx, float y, bool divide) {
+  if (divide) {
+#pragma unroll
+    for (int n = 0; n < 4; ++n) a.v[n] = div_pair(a.v[n], dx);
+    return a;
+  }
+#pragma unroll
+  for (int n = 0; n < 4; ++n)
+    q.v[n] = make_float2(quot_small(a.v[n].x, q.v[n].x, dx, y), quot_small(a.v[n].y, q.v[n].y, dx, y));
+  return q;
+}
+
 // The recurrences of four cells' pairs, psi = b*psi + c*difference/dx, old
 // values in and new ones out.  The quotient is div_by's corrected product,
 // taken for every numerator a on a*2^64: exact where lo2 <= |a| < hi*2^-64,
@@ -319,6 +335,9 @@ __device__ __noinline__ float2 quot_pair(float2 a, float2 q, float dx, float y) 
 // (176x160x129, 200 steps from rest: 143 us a step, from a filled state 84).
 // With the remainder taken as q0*dx - a, zeros come out with their sign too.
 // The rest (subnormal quotients, huge numerators, infinities) goes out of line.
+// ONE: in one call, which takes 1.5 KB less of the loops and more registers
+// across it; the kernels choose by what they measured (kOneCall).
+template <bool ONE>
 __device__ __forceinline__ P4 recur(const fdtd_dev &d, P4 ps, const Q4 &b, const Q4 &c,
                                     const Q4 &da, const Q4 &db) {
   const float2 dx = {d.dx, d.dx}, ny = {-d.rdx, -d.rdx}, s = {-0x1p64f, -0x1p64f};
@@ -336,12 +355,21 @@ __device__ __forceinline__ P4 recur(const fdtd_dev &d, P4 ps, const Q4 &b, const
   float u = 0x1p-64f;
   if (least < __float_as_uint(d.div_lo2) * 2u - 1u || most >= d.div_hi * 0x1p-64f) {
     u = 1.f;
-    if (most >= d.div_hi * 0x1p-64f || d.div_lo > 0x1p-60f) {
+    const bool divide = most >= d.div_hi * 0x1p-64f || d.div_lo > 0x1p-60f;
+    if (ONE) {
+      F8 x, z;
 #pragma unroll
-      for (int n = 0; n < 4; ++n) q[n] = div_pair(a[n], d.dx);
+      for (int n = 0; n < 4; ++n) {
+        x.v[n] = a[n];
+        z.v[n] = q[n];
+      }
+      z = quot_all(x, z, d.dx, d.rdx, divide);
+#pragma unroll
+      for (int n = 0; n < 4; ++n) q[n] = z.v[n];
     } else {
 #pragma unroll
-      for (int n = 0; n < 4; ++n) q[n] = quot_pair(a[n], q[n], d.dx, d.rdx);
+      for (int n = 0; n < 4; ++n)
+        q[n] = divide ? div_pair(a[n], d.dx) : quot_pair(a[n], q[n], d.dx, d.rdx);
     }
   }
 #pragma unroll
@@ -674,6 +702,12 @@ __device__ __noinline__ void gather_probes(const fdtd_dev &d, const int32_t *pz,
   }
 }
 
+// A pair at a time / one call (us a step): mode 1 160^3 61.4/58.7, 192^3
+// 92.9/90.9; coefficient arrays 192^3 133/121, 320^3 530/503, but 128^3 45.3/47.1;
+// mode 5 128^3 49.6/47.2, but 256^3 226/233.
+template <bool OB, bool TAB, bool AHEAD>
+constexpr bool kOneCall = OB ? !AHEAD : (TAB || AHEAD);
+
 // MU: per-cell H coefficients (fdtd_set_magnetic).
 // OB: mode 5.  TAB: material ids with a table that fits shared memory.  One
 // kernel each, since what a step does not need would cost it instruction cache.
@@ -687,6 +721,7 @@ __global__ void __launch_bounds__(kThreads<NG>, 1)
   using L = FG<NG, G>;
   using S = Stage<G>;
   constexpr int ST = L::STAGE;
+  constexpr bool kOne = kOneCall<OB, TAB, AHEAD>;
   float *stab = reinterpret_cast<float *>(smem_all + L::TAB);
   Ctrl *ctrl = reinterpret_cast<Ctrl *>(smem_all + L::CTRL);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -966,7 +1001,7 @@ __global__ void __launch_bounds__(kThreads<NG>, 1)
               put_back(dEx_z, none, past);
             }
             if (sy) {
-              ps = recur(d, ps, all4(tb[py]), all4(tc[py]), dEz_y, dEx_y);
+              ps = recur<kOne>(d, ps, all4(tb[py]), all4(tc[py]), dEz_y, dEx_y);
               corr4<false, 0>(hx, Cx, ps, dx);
               corr4<true, 1>(hz, Cz, ps, dx);
               stp4(psi_pairs(d, PSI_HY) + oy, ps);
@@ -977,7 +1012,7 @@ __global__ void __launch_bounds__(kThreads<NG>, 1)
               const Q4 hy0 = hy, hz0 = hz;
               const uint32_t out =
                   grading_x(tb, tc, i, [&](int v) { return slab_h(v, I, p); }, b, c);
-              ps = recur(d, ps, b, c, dEz_x, dEy_x);
+              ps = recur<kOne>(d, ps, b, c, dEz_x, dEy_x);
               corr4<true, 0>(hy, Cy, ps, dx);
               corr4<false, 1>(hz, Cz, ps, dx);
               put_back(hy, hy0, out);
@@ -987,7 +1022,7 @@ __global__ void __launch_bounds__(kThreads<NG>, 1)
             if (sz) {
               float2 *Z = psi_pairs(d, PSI_HZ) + (oz + pz * plane);
               if (sy || sx) ps = ldp4(Z);
-              ps = recur(d, ps, all4(tb[pz]), all4(tc[pz]), dEy_z, dEx_z);
+              ps = recur<kOne>(d, ps, all4(tb[pz]), all4(tc[pz]), dEy_z, dEx_z);
               corr4<true, 0>(hx, Cx, ps, dx);
               corr4<false, 1>(hy, Cy, ps, dx);
               stp4(Z, ps);
@@ -1139,7 +1174,7 @@ __global__ void __launch_bounds__(kThreads<NG>, 1)
               put_back(dHx_z, none, off);
             }
             if (sy) {
-              ps = recur(d, ps, all4(tb[py]), all4(tc[py]), dHz_y, dHx_y);
+              ps = recur<kOne>(d, ps, all4(tb[py]), all4(tc[py]), dHz_y, dHx_y);
               corr4<true, 0>(ex, Cx, ps, dx);
               corr4<false, 1>(ez, Cz, ps, dx);
               stp4(psi_pairs(d, PSI_EY) + oy, ps);
@@ -1147,7 +1182,7 @@ __global__ void __launch_bounds__(kThreads<NG>, 1)
             if (sz) {
               float2 *Z = psi_pairs(d, PSI_EZ) + (oz + pz * plane);
               if (sy) ps = ldp4(Z);
-              ps = recur(d, ps, all4(tb[pz]), all4(tc[pz]), dHy_z, dHx_z);
+              ps = recur<kOne>(d, ps, all4(tb[pz]), all4(tc[pz]), dHy_z, dHx_z);
               corr4<false, 0>(ex, Cx, ps, dx);
               corr4<true, 1>(ey, Cy, ps, dx);
               stp4(Z, ps);
@@ -1158,7 +1193,7 @@ __global__ void __launch_bounds__(kThreads<NG>, 1)
               const Q4 ey0 = ey, ez0 = ez;
               const uint32_t out =
                   grading_x(tb, tc, i, [&](int v) { return slab_e(v, I, p); }, b, c);
-              ps = recur(d, ps, b, c, dHz_x, dHy_x);
+              ps = recur<kOne>(d, ps, b, c, dHz_x, dHy_x);
               corr4<false, 0>(ey, Cy, ps, dx);
               corr4<true, 1>(ez, Cz, ps, dx);
               put_back(ey, ey0, out);
