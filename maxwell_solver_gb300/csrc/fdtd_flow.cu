@@ -38,7 +38,7 @@
  * 10 % at 256^3 with an oblique wave, and rolled set-up loops, one psi load for
  * three axes and 32-bit cell offsets (75 to 71 KB) 8 % from 96^3 to 192^3.
  *
- * Measured (us a step, separate kernels / this): 64^3 mode 3 27.7/14.3;
+ * Measured (us a step, separate kernels / this): 64^3 mode 3 27.7/13.2;
  * 131x117x109 mode 5 64.8/53.7; 176x160x129 mode 4 with coefficient arrays
  * 120/76; 256^3 mode 5 281/220; 400x360x120 with a current 314/226;
  * 512x512x448 mode 1 1492/1354.  From 256^3 on that is 80-90 % of the measured
@@ -593,6 +593,44 @@ __device__ __forceinline__ void face_pass(const fdtd_dev &d, const float *stab, 
   }
 }
 
+// The corrections of modes 1-4 on a thread's four cells of a plane, within the
+// planes' loop: f the components of H (or E) and C their Che (or Cexh..).  A
+// half-step corrects the two components that are not `only`, each on the faces
+// of the remaining axis.  For grids whose steps are a chain of waits this saves
+// the item's second visit to its cells (us a step, afterwards / here: 48^3
+// 14.4/12.2, 64^3 15.0/13.4); otherwise the code costs more than the visit (96^3
+// 21/28).
+template <bool H>
+__device__ __forceinline__ void axis_faces(const fdtd_dev &d, int mode, const float *row, int i,
+                                           int j, int k, Q4 *const f[3], const Q4 *const C[3]) {
+  const int only = H ? (mode == 2 ? 0 : (mode == 3 ? 2 : 1)) : (mode == 1 ? 0 : (mode == 4 ? 2 : 1));
+  const bool flip = !H && (mode == 2 || mode == 4);
+#pragma unroll
+  for (int t = 0; t < 3; ++t) {
+    if (t == only) continue;
+    const int ax = 3 - t - only, ce = H ? only : t;
+    const bool first = ce == (ax == 2 ? 0 : ax + 1);  // the pair (E_u, H_v)
+    const int lo = pick3(ax, d.i0, d.j0, d.k0), hi = pick3(ax, d.i1, d.j1, d.k1);
+#pragma unroll 1
+    for (int side = 0; side < 2; ++side) {
+      const int own = side ? hi : lo - H;
+      const int a0 = ax == 0 ? own : d.i0, a1 = ax == 0 ? own : d.i1 - (ce == 0);
+      const int b0 = ax == 1 ? own : d.j0, b1 = ax == 1 ? own : d.j1 - (ce == 1);
+      const int c0 = ax == 2 ? own : d.k0, c1 = ax == 2 ? own : d.k1 - (ce == 2);
+      if (j < b0 || j > b1 || k < c0 || k > c1 || i + 3 < a0 || i > a1) continue;
+      const int at = side ? hi : lo - 1 + H;
+      const bool plus = (first == (side == 0)) != flip;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        if (i + e < a0 || i + e > a1) continue;
+        const float v = row[mode < 3 ? (ax == 2 ? at : k) : (ax == 0 ? at : i + e)];
+        const float w = get(*C[t], e) * v;
+        set(*f[t], e, plus ? get(*f[t], e) + w : get(*f[t], e) - w);
+      }
+    }
+  }
+}
+
 // The current source on the item's cells in the box (gpu.h:55-82).
 __device__ __noinline__ void current_pass(const fdtd_dev &d, const fdtd_op &op, int step, Box t,
                                           int tid) {
@@ -711,9 +749,10 @@ constexpr bool kOneCall = OB ? !AHEAD : (TAB || AHEAD);
 // MU: per-cell H coefficients (fdtd_set_magnetic).
 // OB: mode 5.  TAB: material ids with a table that fits shared memory.  One
 // kernel each, since what a step does not need would cost it instruction cache.
-// AHEAD: the pairs of the next plane are brought to L2 a plane ahead, for grids
-// that do not stay there (fdtd_flow::ahead).
-template <int NG, bool MU, bool OB, bool TAB, bool AHEAD, class G>
+// SIZE: big, the pairs of the next plane are brought to L2 a plane ahead, for
+// grids that do not stay there (fdtd_flow::ahead); small, axis_faces.
+constexpr int kSmall = 0, kMid = 1, kBig = 2;
+template <int NG, bool MU, bool OB, bool TAB, int SIZE, class G>
 __global__ void __launch_bounds__(kThreads<NG>, 1)
     k_flow(const __grid_constant__ fdtd_dev d, const __grid_constant__ fdtd_op op,
            const __grid_constant__ FlowMaps mp, const __grid_constant__ Flow f) {
@@ -721,6 +760,7 @@ __global__ void __launch_bounds__(kThreads<NG>, 1)
   using L = FG<NG, G>;
   using S = Stage<G>;
   constexpr int ST = L::STAGE;
+  constexpr bool AHEAD = SIZE == kBig, IN_PLANE = SIZE == kSmall && !OB;
   constexpr bool kOne = kOneCall<OB, TAB, AHEAD>;
   float *stab = reinterpret_cast<float *>(smem_all + L::TAB);
   Ctrl *ctrl = reinterpret_cast<Ctrl *>(smem_all + L::CTRL);
@@ -906,6 +946,12 @@ __global__ void __launch_bounds__(kThreads<NG>, 1)
     // first plane with their plane strides, Z of slab position 0
     const int oz = i + j * d.Ip, plane = (int)d.plane;
     const int sY = 2 * p * d.Ip, sX = fdtd_psi_x_pitch(I, p) * J;
+    // modes 1-4: does the item reach the TF/SF faces (of either kind)?
+    const bool faces =
+        IN_PLANE && op.tfsf_mode && m1.y <= d.i1 && m1.y + G::BX >= d.i0 && m1.z <= d.j1 &&
+        m1.z + G::BY >= d.j0 && kb <= d.k1 && kb + np >= d.k0 &&
+        !(m1.y > d.i0 && m1.y + G::BX <= d.i1 && m1.z > d.j0 && m1.z + G::BY <= d.j1 &&
+          kb > d.k0 && kb + np <= d.k1);
     bool good;
     if (m.x == 0) {
       // ------------------------------------------------------------ H item
@@ -1034,6 +1080,13 @@ __global__ void __launch_bounds__(kThreads<NG>, 1)
               put_back(hz, lds4(sH + 1024), past);
             }
           }
+          if constexpr (IN_PLANE && !kCurl) {
+            if (faces && nv > 0) {
+              Q4 *const ff[3] = {&hx, &hy, &hz};
+              const Q4 *const cc[3] = {&Cx, &Cy, &Cz};
+              axis_faces<true>(d, op.tfsf_mode, inc_h_row(d, op.tfsf_mode, step), i, j, k, ff, cc);
+            }
+          }
           if (kCurl || nv > 0) {
             stg4(d.f[3] + n, hx);
             stg4(d.f[4] + n, hy);
@@ -1050,7 +1103,7 @@ __global__ void __launch_bounds__(kThreads<NG>, 1)
         }
         return true;
       };
-      good = __all_sync(0xffffffffu, nv == 4 && !sy && !sx) && kb >= p && k1 < K - p
+      good = __all_sync(0xffffffffu, nv == 4 && !sy && !sx) && !faces && kb >= p && k1 < K - p
                  ? planes(std::true_type{})
                  : planes(std::false_type{});
     } else {
@@ -1207,6 +1260,13 @@ __global__ void __launch_bounds__(kThreads<NG>, 1)
               put_back(ez, lds4(sE + 1024), past);
             }
           }
+          if constexpr (IN_PLANE && !kCurl) {
+            if (faces && nv > 0) {
+              Q4 *const ff[3] = {&ex, &ey, &ez};
+              const Q4 *const cc[3] = {&Cx, &Cy, &Cz};
+              axis_faces<false>(d, op.tfsf_mode, inc_e_row(d, op.tfsf_mode, step), i, j, k, ff, cc);
+            }
+          }
           if (kCurl || nv > 0) {
             stg4(d.f[0] + n, ex);
             stg4(d.f[1] + n, ey);
@@ -1223,8 +1283,8 @@ __global__ void __launch_bounds__(kThreads<NG>, 1)
         }
         return true;
       };
-      good = __all_sync(0xffffffffu, nv == 4 && py < 0 && !sx_ && i > 0 && j > 0) && kb >= p &&
-                     kb + np <= K - p
+      good = __all_sync(0xffffffffu, nv == 4 && py < 0 && !sx_ && i > 0 && j > 0) && !faces &&
+                     kb >= p && kb + np <= K - p
                  ? planes(std::true_type{})
                  : planes(std::false_type{});
     }
@@ -1235,7 +1295,7 @@ __global__ void __launch_bounds__(kThreads<NG>, 1)
     // the item's face cells, then its source cells
     const Box t = {m1.y, m1.y + G::BX - 1, m1.z, m1.z + G::BY - 1, kb, kb + np - 1};
     bool ok = true;
-    if (op.tfsf_mode) {
+    if (!IN_PLANE && op.tfsf_mode) {
       const uint32_t mask = __ballot_sync(
           0xffffffffu, lane < 12 && face_of<OB>(d, m.x == 0, op.tfsf_mode, lane, t).any);
       if (mask) {
@@ -1274,14 +1334,14 @@ int prepare(K kern, int threads, int smem, int *cached) {
   return 0;
 }
 
-template <bool MU, bool OB, bool TAB, bool AHEAD, class G>
+template <bool MU, bool OB, bool TAB, int SIZE, class G>
 int launch(const fdtd_dev *d, const fdtd_maps_flow *m, const fdtd_op *op, const fdtd_flow *w,
            cudaStream_t s) {
   static_assert(sizeof(FlowMaps) == sizeof(((fdtd_maps_flow *)0)->bytes), "map layout");
   static int cached = 0;
-  constexpr int NG = kGroups<MU, AHEAD>;
+  constexpr int NG = kGroups<MU, SIZE == kBig>;
   constexpr int smem = FG<NG, G>::SMEM;
-  auto kern = k_flow<NG, MU, OB, TAB, AHEAD, G>;
+  auto kern = k_flow<NG, MU, OB, TAB, SIZE, G>;
   if (const int e = prepare(kern, kThreads<NG>, smem, &cached)) return e;
   FlowMaps mp;
   memcpy(&mp, m->bytes, sizeof(FlowMaps));
@@ -1322,9 +1382,11 @@ int launch(const fdtd_dev *d, const fdtd_maps_flow *m, const fdtd_op *op, const 
 template <bool MU, bool OB, bool TAB>
 int launch_tiled(const fdtd_dev *d, const fdtd_maps_flow *m, const fdtd_op *op, const fdtd_flow *w,
                  cudaStream_t s) {
-  if (w->tile == 0) return launch<MU, OB, TAB, true, GS>(d, &m[0], op, w, s);
-  return w->ahead ? launch<MU, OB, TAB, true, GB>(d, &m[1], op, w, s)
-                  : launch<MU, OB, TAB, false, GB>(d, &m[1], op, w, s);
+  if (w->tile == 0) return launch<MU, OB, TAB, kBig, GS>(d, &m[0], op, w, s);
+  if (w->ahead) return launch<MU, OB, TAB, kBig, GB>(d, &m[1], op, w, s);
+  if (!OB && w->zc == 1 && op->tfsf_mode)
+    return launch<MU, OB, TAB, OB ? kMid : kSmall, GB>(d, &m[1], op, w, s);
+  return launch<MU, OB, TAB, kMid, GB>(d, &m[1], op, w, s);
 }
 template <bool MU, bool OB>
 int launch_coef(const fdtd_dev *d, const fdtd_maps_flow *m, const fdtd_op *op, const fdtd_flow *w,
