@@ -3194,13 +3194,13 @@ static int batch_list(batch *b) {
     if (!s) return fail(FDTD_ERR_INVALID_HANDLE, "a batch member was deleted");
     b->act[b->n_act++] = i;
   }
-  /* On their own SMs the members need several each: with fewer, rounding the
-   * shares to whole SMs and the rate of one SM on a small grid cost more than
-   * the launches.  300 steps of members of 32..128 cells a side, mode 5, separate
-   * kernels / multi-step launches (ms): 4 members 29.6/18.4, 8 48.7/40.3, 16
-   * 53.3/42.6, 20 73.2/62.2, 24 94.0/97.0, 32 104/109; 600 steps of 48 293/357.
-   * 100..200 cells, mode 1, 100 steps: 4 39.2/23.0, 16 86.1/74.0. */
-  b->flow = b->n_act * 7 <= sm_count();
+  /* On their own SMs the members need four each: with fewer, rounding the shares
+   * to whole SMs and the rate of one SM on a small grid cost more than the
+   * launches.  300 steps of members of 32..128 cells a side, mode 5, separate
+   * kernels / multi-step launches (ms): 4 members 29.6/17.1, 8 48.7/36.5, 16
+   * 53.3/40.2, 24 94.7/91.0, 32 105/101, 40 120/121, 48 149/169; 32..56 a side:
+   * 24 28.2/22.5, 40 41.7/35.7; 100..160, mode 1, 60 steps: 32 67.3/62.9. */
+  b->flow = b->n_act * 4 <= sm_count();
   for (int g = 0; g < b->n_act && b->flow; ++g) {
     const bmember *m = &b->m[b->act[g]];
     b->flow = flow_possible(lookup(m->h), m->mode, m->has_cur ? &m->cur : NULL);

@@ -107,7 +107,7 @@ def test_multi_step_launches_equal_oracle(name, monkeypatch):
 
 
 def test_batch_changing_route_equals_alone():
-    """24 members run as batched half-steps; as members finish, the 21 and fewer
+    """42 members run as batched half-steps; as members finish, the 38 and fewer
     left go on as multi-step launches; a member added then starts there."""
     from maxwell_solver_gb300 import simFDTD
     from maxwell_solver_gb300.batch import Batch
@@ -123,15 +123,15 @@ def test_batch_changing_route_equals_alone():
     def current(sc):
         return (sc.cur_mode, sc.cur_box) if sc.cur_mode else None
 
-    mix = [SCENARIOS[g % len(SCENARIOS)] for g in range(25)]
-    steps = [20 + g for g in range(25)]
+    mix = [SCENARIOS[g % len(SCENARIOS)] for g in range(43)]
+    steps = [10 + g for g in range(43)]
     members = [ready(sc) for sc in mix]
     with Batch() as b:
-        for P, sc, n in zip(members[:24], mix, steps):
+        for P, sc, n in zip(members[:42], mix, steps):
             b.add(P, 0, n, sc.mode, current(sc))
-        for _ in range(5):  # to the end of the first members, and past it
+        for _ in range(8):  # past the change of route
             b.step(1 << 20)
-        b.add(members[24], 0, steps[24], mix[24].mode, current(mix[24]))
+        b.add(members[42], 0, steps[42], mix[42].mode, current(mix[42]))
         b.step(3)
         b.run()
         for P, sc, n in zip(members, mix, steps):
