@@ -206,9 +206,10 @@ typedef struct {
 
 /* Runs steps first..first+count-1 of the reference step order
  * (highfrequency.m:85-91, plus AddCurrents as in GICsimulation.m:119-124
- * when cur != NULL and cur->mode != 0), each step as two fused half-step
- * kernels, with the loop captured in a CUDA graph.  tfsf_mode 0 skips the
- * plane-wave corrections.  Bitwise identical to issuing the per-op calls. */
+ * when cur != NULL and cur->mode != 0), many steps per launch; steps that
+ * cannot run so take two fused half-step kernels each, the loop captured in a
+ * CUDA graph.  tfsf_mode 0 skips the plane-wave corrections.  Bitwise
+ * identical to issuing the per-op calls. */
 int fdtd_step_n(fdtd_handle h, int32_t first, int32_t count, int32_t tfsf_mode,
                 const fdtd_current *cur);
 
@@ -277,8 +278,9 @@ int fdtd_set_device(int32_t device);
 /* ---------------------------------------------------------------------
  * Batched execution (extension, no reference counterpart): many ready
  * simulation handles of different sizes, materials and sources advance
- * together, one H and one E launch per step for all of them (persistent
- * TMA kernels over the work items of every member).  The arithmetic per
+ * together: each on its share of the GPU, or with many members one H and one
+ * E launch per step for all of them (persistent TMA kernels over the work
+ * items of every member).  The arithmetic per
  * cell is unchanged: each member ends bit-identical to running it alone.
  * --------------------------------------------------------------------- */
 typedef uint64_t fdtd_batch;
