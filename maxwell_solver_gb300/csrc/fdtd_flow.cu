@@ -658,6 +658,8 @@ __device__ __noinline__ void current_pass(const fdtd_dev &d, const fdtd_op &op, 
 // the item's row counter is raised with gpu-scope release, so that the
 // consumers never wait for their stores to land.  Gives up without progress
 // for twice the waits' limit, or when a block has reported an error.
+// Polling without a pause between costs the others nothing measurable and gains
+// 1-2 % up to 200^3 (131x117x109 52.9 -> 52.0 us a step, 128^3 36.7 -> 35.8).
 template <int NG>
 __device__ __forceinline__ void release_items(Ctrl *ctrl, uint32_t *cnt, const int32_t *err,
                                               int lane) {
@@ -681,8 +683,6 @@ __device__ __forceinline__ void release_items(Ctrl *ctrl, uint32_t *cnt, const i
         }
       }
       t0 = global_ns();
-    } else {
-      __nanosleep(32);  // leave the issue slots to the others
     }
     if ((it & 1023u) == 0u) {
       const bool bad = global_ns() - t0 > 2 * kWaitNs || (err && *(const volatile int32_t *)err);
