@@ -171,6 +171,7 @@ typedef struct sim {
   /* many steps per launch (fdtd_flow.cu): the row counters, the steps they
    * have counted since they were zeroed and the item height they were zeroed
    * for (0: not zeroed), the item geometry, and the probes by z-plane */
+  int32_t *d_flow_mem, *h_flow; /* what follows is in d_flow_mem */
   uint32_t *d_flow;
   uint32_t flow_base;
   int32_t flow_counted;
@@ -438,9 +439,8 @@ int fdtd_destroy(fdtd_handle h) {
   dfree(s->d_hrep);
   dfree(s->d_hid);
   dfree(s->d_hcnt);
-  dfree(s->d_flow);
-  dfree(s->d_pz);
-  dfree(s->d_pat);
+  dfree(s->d_flow_mem);
+  free(s->h_flow);
   free(s->h_src);
   free(s->h_probe_idx);
   free(s->h_den_ex);
@@ -1211,9 +1211,6 @@ static int fused_mode(void) {
  * z-plane. */
 #define FLOW_BIG 4000000 /* cells */
 static int flow_setup(sim *s) {
-  int rc;
-  const int64_t n = fdtdk_flow_counters(s->J, s->K);
-  if ((rc = dalloc(s, (void **)&s->d_flow, (size_t)n * sizeof(uint32_t)))) return rc;
   s->flow_counted = 0;
   /* Item height: a half-step should have an item or more for each of the
    * 456 groups (3 on each of 152 SMs), then as many planes as that leaves,
@@ -1236,18 +1233,26 @@ static int flow_setup(sim *s) {
   s->flow_tile = big && s->I >= 320 ? 0 : 1;
   s->flow_zc = s->cells < 350000 ? 1 : s->cells < 1100000 ? 2 : big ? 8 : 4;
   if (s->flow_zc > s->K) s->flow_zc = s->K;
+  /* one allocation: the probes by plane, each plane's first, the counters */
+  const int K = s->K, probes = s->init_ant && s->num_ant > 0 ? s->num_ant : 0;
+  const size_t lists = probes ? 4 * (size_t)probes + (((size_t)K + 1 + 3) & ~(size_t)3) : 0;
+  const size_t counters = (size_t)fdtdk_flow_counters(s->J, K);
+  int rc = dalloc(s, (void **)&s->d_flow_mem, (lists + counters) * sizeof(int32_t));
+  if (rc) return rc;
+  s->d_flow = (uint32_t *)(s->d_flow_mem + lists);
   s->n_pat = 0;
-  if (!s->init_ant || s->num_ant <= 0) return FDTD_OK;
-  const int K = s->K;
-  int32_t *pz = (int32_t *)calloc((size_t)K + 1, sizeof(int32_t));
-  int32_t *pat = (int32_t *)calloc((size_t)s->num_ant * 4, sizeof(int32_t));
+  if (!probes) return FDTD_OK;
+  s->d_pat = s->d_flow_mem;
+  s->d_pz = s->d_flow_mem + 4 * (size_t)probes;
+  /* kept until the handle goes: the copy below may still read it */
+  free(s->h_flow);
+  s->h_flow = (int32_t *)calloc(lists, sizeof(int32_t));
   int32_t *at = (int32_t *)calloc((size_t)K, sizeof(int32_t));
-  if (!pz || !pat || !at) {
-    free(pz);
-    free(pat);
+  if (!s->h_flow || !at) {
     free(at);
     return fail(FDTD_ERR_OOM, "out of host memory");
   }
+  int32_t *pat = s->h_flow, *pz = s->h_flow + 4 * (size_t)probes;
   /* a probe belongs to the H item whose cells hold it, the last plane, row
    * and column to the ones before them */
   for (int pass = 0; pass < 2; ++pass) {
@@ -1271,20 +1276,10 @@ static int flow_setup(sim *s) {
     if (pass == 0)
       for (int k = 0; k < K; ++k) pz[k + 1] += pz[k];
   }
-  const size_t zb = ((size_t)K + 1) * sizeof(int32_t), ab = (size_t)s->num_ant * 4 * sizeof(int32_t);
-  if (!(rc = dalloc(s, (void **)&s->d_pz, zb))) rc = dalloc(s, (void **)&s->d_pat, ab);
-  cudaError_t e = cudaSuccess;
-  if (!rc) {
-    e = cudaMemcpyAsync(s->d_pz, pz, zb, cudaMemcpyHostToDevice, s->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(s->d_pat, pat, ab, cudaMemcpyHostToDevice, s->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
-    if (s->n_pat == 0) s->n_pat = s->num_ant;
-  }
-  free(pz);
-  free(pat);
   free(at);
-  if (rc) return rc;
-  CU(e);
+  if (s->n_pat == 0) s->n_pat = s->num_ant;
+  CU(cudaMemcpyAsync(s->d_flow_mem, s->h_flow, lists * sizeof(int32_t), cudaMemcpyHostToDevice,
+                     s->stream));
   return FDTD_OK;
 }
 
@@ -2502,7 +2497,7 @@ int fdtd_estimate_device_bytes(int32_t I, int32_t J, int32_t K, int32_t pml, int
   b += (uint64_t)HASH_CAP * (8 + 8 + 4) + 16 + 4;  /* indexing scratch, error word */
   b += 2 * psi * 4;                                /* psi pairs */
   b += (uint64_t)fdtdk_flow_counters(J, K) * 4 +
-       ((uint64_t)K + 1 + 4 * (uint64_t)num_ant) * 4; /* multi-step counters, probe lists */
+       ((uint64_t)K + 4 + 4 * (uint64_t)num_ant) * 4; /* multi-step counters, probe lists */
   if (fused_mode() == 1 || (fused_mode() < 0 && tune_enabled() &&
                               (int64_t)cells >= TUNE_MIN_CELLS))
     b += 6 * cells * 4 + psi * 4;                  /* the fused step's second buffer
