@@ -631,6 +631,38 @@ __device__ __forceinline__ void axis_faces(const fdtd_dev &d, int mode, const fl
   }
 }
 
+// The same for mode 5: component t is corrected on the faces of the other two
+// axes in their order, which is the order of ob_plane's owner (us a step,
+// afterwards / here: 24^3 37/19, 48^3 25/19, 64^3 26/20; 96^3 at two planes an
+// item 35/39).  The cells go one by one, which keeps the code small.
+template <bool H>
+__device__ __forceinline__ void oblique_faces(const fdtd_dev &d, const float *row, int i, int j,
+                                              int k, Q4 *const f[3], const Q4 *const C[3]) {
+#pragma unroll
+  for (int t = 0; t < 3; ++t) {
+#pragma unroll 1
+    for (int face = 0; face < 4; ++face) {
+      const int side = face & 1, ax = face < 2 ? (t == 0 ? 1 : 0) : (t == 2 ? 1 : 2);
+      const int ce = H ? 3 - ax - t : t, ch = H ? t : 3 - ax - t;
+      const bool first = ce == (ax == 2 ? 0 : ax + 1);  // the pair (E_u, H_v)
+      const int lo = pick3(ax, d.i0, d.j0, d.k0), hi = pick3(ax, d.i1, d.j1, d.k1);
+      const int own = side ? hi : lo - H;
+      const int a0 = ax == 0 ? own : d.i0, a1 = ax == 0 ? own : d.i1 - (ce == 0);
+      const int b0 = ax == 1 ? own : d.j0, b1 = ax == 1 ? own : d.j1 - (ce == 1);
+      const int c0 = ax == 2 ? own : d.k0, c1 = ax == 2 ? own : d.k1 - (ce == 2);
+      if (j < b0 || j > b1 || k < c0 || k > c1) continue;
+      const bool plus = first == (side == 0);
+#pragma unroll 1
+      for (int e = max(a0 - i, 0); e <= min(a1 - i, 3); ++e) {
+        const float w = get(*C[t], e) * incident<true>(d, H, FDTD_MODE_OBLIQUE, row, ax, side, ce,
+                                                       ch, i + e, j, k);
+        const float v = get(*f[t], e);
+        set(*f[t], e, plus ? v + w : v - w);
+      }
+    }
+  }
+}
+
 // The current source on the item's cells in the box (gpu.h:55-82).
 __device__ __noinline__ void current_pass(const fdtd_dev &d, const fdtd_op &op, int step, Box t,
                                           int tid) {
@@ -750,7 +782,8 @@ constexpr bool kOneCall = OB ? !AHEAD : (TAB || AHEAD);
 // OB: mode 5.  TAB: material ids with a table that fits shared memory.  One
 // kernel each, since what a step does not need would cost it instruction cache.
 // SIZE: big, the pairs of the next plane are brought to L2 a plane ahead, for
-// grids that do not stay there (fdtd_flow::ahead); small, axis_faces.
+// grids that do not stay there (fdtd_flow::ahead); small, axis_faces and
+// oblique_faces.
 constexpr int kSmall = 0, kMid = 1, kBig = 2;
 template <int NG, bool MU, bool OB, bool TAB, int SIZE, class G>
 __global__ void __launch_bounds__(kThreads<NG>, 1)
@@ -760,7 +793,7 @@ __global__ void __launch_bounds__(kThreads<NG>, 1)
   using L = FG<NG, G>;
   using S = Stage<G>;
   constexpr int ST = L::STAGE;
-  constexpr bool AHEAD = SIZE == kBig, IN_PLANE = SIZE == kSmall && !OB;
+  constexpr bool AHEAD = SIZE == kBig, IN_PLANE = SIZE == kSmall;
   constexpr bool kOne = kOneCall<OB, TAB, AHEAD>;
   float *stab = reinterpret_cast<float *>(smem_all + L::TAB);
   Ctrl *ctrl = reinterpret_cast<Ctrl *>(smem_all + L::CTRL);
@@ -946,7 +979,7 @@ __global__ void __launch_bounds__(kThreads<NG>, 1)
     // first plane with their plane strides, Z of slab position 0
     const int oz = i + j * d.Ip, plane = (int)d.plane;
     const int sY = 2 * p * d.Ip, sX = fdtd_psi_x_pitch(I, p) * J;
-    // modes 1-4: does the item reach the TF/SF faces (of either kind)?
+    // does the item reach the TF/SF faces (of either kind)?
     const bool faces =
         IN_PLANE && op.tfsf_mode && m1.y <= d.i1 && m1.y + G::BX >= d.i0 && m1.z <= d.j1 &&
         m1.z + G::BY >= d.j0 && kb <= d.k1 && kb + np >= d.k0 &&
@@ -1084,7 +1117,10 @@ __global__ void __launch_bounds__(kThreads<NG>, 1)
             if (faces && nv > 0) {
               Q4 *const ff[3] = {&hx, &hy, &hz};
               const Q4 *const cc[3] = {&Cx, &Cy, &Cz};
-              axis_faces<true>(d, op.tfsf_mode, inc_h_row(d, op.tfsf_mode, step), i, j, k, ff, cc);
+              if constexpr (OB)
+                oblique_faces<true>(d, d.ob_inc[0] + (int64_t)step * d.ob_w, i, j, k, ff, cc);
+              else
+                axis_faces<true>(d, op.tfsf_mode, inc_h_row(d, op.tfsf_mode, step), i, j, k, ff, cc);
             }
           }
           if (kCurl || nv > 0) {
@@ -1264,7 +1300,10 @@ __global__ void __launch_bounds__(kThreads<NG>, 1)
             if (faces && nv > 0) {
               Q4 *const ff[3] = {&ex, &ey, &ez};
               const Q4 *const cc[3] = {&Cx, &Cy, &Cz};
-              axis_faces<false>(d, op.tfsf_mode, inc_e_row(d, op.tfsf_mode, step), i, j, k, ff, cc);
+              if constexpr (OB)
+                oblique_faces<false>(d, d.ob_inc[1] + (int64_t)step * d.ob_w, i, j, k, ff, cc);
+              else
+                axis_faces<false>(d, op.tfsf_mode, inc_e_row(d, op.tfsf_mode, step), i, j, k, ff, cc);
             }
           }
           if (kCurl || nv > 0) {
@@ -1384,8 +1423,7 @@ int launch_tiled(const fdtd_dev *d, const fdtd_maps_flow *m, const fdtd_op *op, 
                  cudaStream_t s) {
   if (w->tile == 0) return launch<MU, OB, TAB, kBig, GS>(d, &m[0], op, w, s);
   if (w->ahead) return launch<MU, OB, TAB, kBig, GB>(d, &m[1], op, w, s);
-  if (!OB && w->zc == 1 && op->tfsf_mode)
-    return launch<MU, OB, TAB, OB ? kMid : kSmall, GB>(d, &m[1], op, w, s);
+  if (w->zc == 1 && op->tfsf_mode) return launch<MU, OB, TAB, kSmall, GB>(d, &m[1], op, w, s);
   return launch<MU, OB, TAB, kMid, GB>(d, &m[1], op, w, s);
 }
 template <bool MU, bool OB>

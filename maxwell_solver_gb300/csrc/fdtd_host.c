@@ -2272,21 +2272,13 @@ static int run_fused(sim *s, int32_t first, int32_t count, int32_t mode) {
 }
 
 /* Can steps of this mode (and current) run as multi-step launches? */
-static int flow_possible(sim *s, int32_t mode, const fdtd_current *cur) {
+static int flow_usable(sim *s, int32_t mode, const fdtd_current *cur) {
   if (!s->use_tma || !s->maps[0].valid || !s->d_flow || s->n_pat < 0) return 0;
   if (!s->wmaps[s->flow_tile].valid) return 0;
   if (s->dev.num_ant > 0 && s->n_pat == 0) return 0;
   fdtd_op o;
   step_op_e(&o, mode, cur);
   return fdtd_flow_ok(&s->dev, &o);
-}
-
-/* Mode 5 corrects every component on all six faces.  On a tiny grid of its own
- * that is most of an item's time, and separate kernels spread it better (us a
- * step, separate / this way: 24^3 24/35, 48^3 31/26, 64^3 27/27, 96^3 50/37). */
-#define FLOW_MIN_OBLIQUE 65536 /* cells */
-static int flow_usable(sim *s, int32_t mode, const fdtd_current *cur) {
-  return (mode != FDTD_MODE_OBLIQUE || s->cells >= FLOW_MIN_OBLIQUE) && flow_possible(s, mode, cur);
 }
 
 /* n steps from `first` on the handle's stream, zc planes an item; on at most
@@ -2337,7 +2329,7 @@ static int run_steps(sim *s, int32_t first, int32_t count, int32_t mode,
   const int probes = s->dev.num_ant > 0;
   int32_t done = 0;
   /* Multi-step launches unless FDTD_FUSED=1 asked for the fused pairs: they
-   * are faster than either other way at every size measured (flow_usable). */
+   * are faster than either other way at every size measured (24^3 to 512^3). */
   const int forced = s->fused_forced && fused_usable(s, mode, cur);
   if (!forced && flow_usable(s, mode, cur))
     return run_flow(s, first, count, mode, cur, s->flow_zc, 0, s->d_err);
@@ -3198,7 +3190,7 @@ static int batch_list(batch *b) {
   b->flow = b->n_act * 4 <= sm_count();
   for (int g = 0; g < b->n_act && b->flow; ++g) {
     const bmember *m = &b->m[b->act[g]];
-    b->flow = flow_possible(lookup(m->h), m->mode, m->has_cur ? &m->cur : NULL);
+    b->flow = flow_usable(lookup(m->h), m->mode, m->has_cur ? &m->cur : NULL);
   }
   b->mirrored = 0;
   b->dirty = 0;

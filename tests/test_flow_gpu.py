@@ -24,6 +24,8 @@ CASES = {
     "huge": ((50, 41, 33), 7, 9, 60, 3, "current 1e24"),
     "plain_current": ((63, 47, 35), 8, 10, 40, 0, "current arrays"),
     "oblique": ((71, 38, 43), 6, 8, 60, 5, "arrays"),
+    "oblique_small": ((33, 41, 35), 5, 7, 60, 5, "magnetic"),
+    "oblique_over_tiles": ((65, 49, 34), 8, 10, 60, 5, ""),
     "oblique_two_planes": ((97, 73, 66), 9, 11, 60, 5, "magnetic"),
     "oblique_four_planes": ((130, 117, 109), 9, 11, 60, 5, ""),
     "two_planes": ((97, 81, 67), 10, 12, 48, 3, "current"),
