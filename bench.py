@@ -553,7 +553,7 @@ def run_batched(n_grids: int, batched_only: bool = False):
     t_one = t_ops = None
     ref = {}
     if not batched_only:
-        # one at a time through fdtd_step_n (graph-replayed fused steps)
+        # one at a time through fdtd_step_n (multi-step launches)
         t0 = time.perf_counter()
         for P, s in zip(handles, mix):
             simFDTD("StepN", P, np.int32([0, s.steps, s.mode]))
@@ -612,7 +612,7 @@ def run_batched(n_grids: int, batched_only: bool = False):
         "zrun": zrun,
         "identical_results": bool(same), "members_compared": len(ref),
         "timing": "wall clock, fields resident, setup excluded; one at a time = fdtd_step_n "
-                  "per grid (graph-replayed fused steps) and, separately, the per-op calls",
+                  "per grid (multi-step launches) and, separately, the per-op calls",
     }
 
 
