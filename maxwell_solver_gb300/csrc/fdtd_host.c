@@ -1906,6 +1906,22 @@ int fdtd_inject_device_error(fdtd_handle h, int32_t value) {
 static int run_steps(sim *s, int32_t first, int32_t count, int32_t mode,
                      const fdtd_current *cur);
 
+/* The op's current source: the caller's mode and box, clipped to the grid
+ * (the cells of a box that lie outside it take nothing, and the kernels step
+ * through the box).  None when a bound is negative or no cell is left. */
+static void set_current(const sim *s, fdtd_op *o, int32_t mode, const int32_t box[6]) {
+  const int32_t n[3] = {s->I, s->J, s->K};
+  o->cur_mode = 0;
+  if (mode < 1 || mode > 3) return;
+  for (int a = 0; a < 3; ++a) {
+    const int32_t lo = box[2 * a], hi = box[2 * a + 1] < n[a] ? box[2 * a + 1] : n[a] - 1;
+    if (lo < 0 || hi < lo) return;
+    o->cur_box[2 * a] = lo;
+    o->cur_box[2 * a + 1] = hi;
+  }
+  o->cur_mode = mode;
+}
+
 /* A half-step of a whole step: curl, CPML and the step's TF/SF and current
  * source (if any). */
 static int whole_half(const fdtd_op *o) {
@@ -2133,42 +2149,29 @@ int fdtd_add_currents(fdtd_handle h, int32_t step, int32_t mode, const int32_t b
   if (!s->init_src) return fail(FDTD_ERR_STATE, "AddCurrents requires SetSource");
   if (step < 0 || step >= s->T)
     return fail(FDTD_ERR_INVALID_ARG, "time step %d outside [0, %d)", step, s->T);
-  if (mode < 1 || mode > 3) return FDTD_OK;
-  for (int a = 0; a < 6; ++a)
-    if (box[a] < 0) return FDTD_OK; /* reference: no cell is touched */
-  if (box[1] < box[0] || box[3] < box[2] || box[5] < box[4]) return FDTD_OK;
   fdtd_op st;
   memset(&st, 0, sizeof(st));
-  st.cur_mode = mode;
-  memcpy(st.cur_box, box, sizeof(st.cur_box));
+  set_current(s, &st, mode, box);
+  if (!st.cur_mode) return FDTD_OK; /* as the reference: no cell is touched */
   st.step = step;
   return enqueue(s, 0, 4, &st);
 }
 
 /* ------------------------------------------------------------ fused loop */
 
-/* The E half-step of a whole step: curl, CPML, TF/SF mode, current source
- * (none when its box is empty or negative: the reference touches no cell). */
-static void step_op_e(fdtd_op *o, int32_t mode, const fdtd_current *cur) {
+/* The E half-step of a whole step: curl, CPML, TF/SF mode, current source. */
+static void step_op_e(const sim *s, fdtd_op *o, int32_t mode, const fdtd_current *cur) {
   memset(o, 0, sizeof(*o));
   o->curl = 1;
   o->pml = 1;
   o->tfsf_mode = mode;
-  if (cur && cur->mode >= 1 && cur->mode <= 3) {
-    int ok = 1;
-    for (int a = 0; a < 6; ++a) ok &= cur->box[a] >= 0;
-    ok &= cur->box[1] >= cur->box[0] && cur->box[3] >= cur->box[2] && cur->box[5] >= cur->box[4];
-    if (ok) {
-      o->cur_mode = cur->mode;
-      memcpy(o->cur_box, cur->box, sizeof(o->cur_box));
-    }
-  }
+  if (cur) set_current(s, o, cur->mode, cur->box);
 }
 
 static int step_ops(sim *s, int32_t step, int from_dev, int32_t mode, const fdtd_current *cur) {
   fdtd_op oh, oe;
-  step_op_e(&oe, mode, cur);
-  step_op_e(&oh, mode, NULL);
+  step_op_e(s, &oe, mode, cur);
+  step_op_e(s, &oh, mode, NULL);
   oh.step = oe.step = step;
   oh.step_from_dev = oe.step_from_dev = from_dev;
   if (s->dev.num_ant > 0) KL(fdtdk_probe_gather(&s->dev, s->stream));
@@ -2277,7 +2280,7 @@ static int flow_usable(sim *s, int32_t mode, const fdtd_current *cur) {
   if (!s->wmaps[s->flow_tile].valid) return 0;
   if (s->dev.num_ant > 0 && s->n_pat == 0) return 0;
   fdtd_op o;
-  step_op_e(&o, mode, cur);
+  step_op_e(s, &o, mode, cur);
   return fdtd_flow_ok(&s->dev, &o);
 }
 
@@ -2305,7 +2308,7 @@ static int run_flow(sim *s, int32_t first, int32_t count, int32_t mode, const fd
     w.n_probes = s->n_pat;
   }
   fdtd_op o;
-  step_op_e(&o, mode, cur);
+  step_op_e(s, &o, mode, cur);
   /* A launch lasts some 10 ms at most, so that other streams' work gets its
    * turn; its tickets then fit their 32-bit counter many times over. */
   const int64_t cs = (int64_t)1 << (blocks ? 31 : 29);
@@ -2430,10 +2433,7 @@ int fdtd_profile_steps(fdtd_handle h, int32_t first, int32_t count, int32_t mode
     oh.tfsf_mode = mode;
     oh.step = first + c;
     oe = oh;
-    if (use_cur) {
-      oe.cur_mode = cur->mode;
-      memcpy(oe.cur_box, cur->box, sizeof(oe.cur_box));
-    }
+    if (use_cur) set_current(s, &oe, cur->mode, cur->box);
     /* ev[12] / ev[13]: recorded right after the H / E curl kernel (the
      * mark stays at the half-step's start when no curl kernel runs) */
     CU(cudaEventRecord(ev[8], s->stream));
@@ -2975,15 +2975,11 @@ int fdtd_batch_add(fdtd_batch bh, fdtd_handle h, int32_t first, int32_t count, i
   m->first = first;
   m->count = count;
   m->mode = mode;
-  m->has_cur = 0;
   if (use_cur) {
-    int ok = 1;
-    for (int a = 0; a < 6; ++a) ok &= cur->box[a] >= 0;
-    ok &= cur->box[1] >= cur->box[0] && cur->box[3] >= cur->box[2] && cur->box[5] >= cur->box[4];
-    if (ok) {
-      m->has_cur = 1;
-      m->cur = *cur;
-    }
+    fdtd_op o;
+    set_current(s, &o, cur->mode, cur->box);
+    m->has_cur = o.cur_mode != 0;
+    m->cur = *cur;
   }
   b->dirty = 1;
   return FDTD_OK;
@@ -3107,10 +3103,7 @@ static int batch_rebuild_(batch *b) {
     op->curl = 1;
     op->pml = 1;
     op->tfsf_mode = m->mode;
-    if (m->has_cur) {
-      op->cur_mode = m->cur.mode;
-      memcpy(op->cur_box, m->cur.box, sizeof(op->cur_box));
-    }
+    if (m->has_cur) set_current(s, op, m->cur.mode, m->cur.box);
     op->tfsf_split = fdtd_tfsf_split(&s->dev, op);
     op->xsplit = xsplit_enabled() && fdtd_xsplit(&s->dev, op);
     if (op->xsplit) {

@@ -147,7 +147,7 @@ typedef struct {
   int32_t step;             /* step index (offset when step_from_dev) */
   int32_t step_from_dev;    /* step = *step_base + step */
   int32_t cur_mode;         /* 0 none, 1..3 Ex/Ey/Ez current source */
-  int32_t cur_box[6];
+  int32_t cur_box[6];       /* its cells, within the grid: bounds inclusive */
   int32_t tfsf_split;       /* TMA kernels: TF/SF applied by the face pass */
   int32_t xsplit;           /* TMA E kernel: CPML X applied by the x-slab pass */
   int32_t pad_[2];
