@@ -112,3 +112,29 @@ def test_box_past_the_grid_is_clipped(name, run):
     _assert_equal(P, o, dims)
     assert (max(np.abs(o.field(f)).max() for f in FIELDS) > 0) == ("outside" not in name)
     simFDTD("DeleteSimulation", P)
+
+
+# The edge j = J-1, k = K-1 in items of its own: J-1 and K-1 multiples of the
+# tile's height and of the item's planes (1, 2, 4 and 8 by grid size; tiles of
+# 16 rows, of 8 for rows of 320 cells and more).  Only the source reaches it.
+EDGE = {
+    "one_plane": ((24, 33, 24), (8, 11, 30, 32, 20, 23)),
+    "one_plane_64": ((64, 65, 64), (5, 40, 64, 64, 63, 63)),
+    "two_planes": ((97, 81, 67), (0, 96, 79, 80, 64, 66)),
+    "four_planes": ((129, 97, 93), (64, 66, 96, 96, 90, 92)),
+    "eight_planes": ((198, 161, 129), (100, 140, 160, 160, 126, 128)),
+    "wide": ((331, 113, 113), (300, 330, 110, 112, 112, 112)),
+}
+
+
+@pytest.mark.parametrize("name", EDGE)
+def test_source_over_the_outer_edge(name):
+    from maxwell_solver_gb300 import simFDTD
+
+    dims, box = EDGE[name]
+    P = _ready(dims)
+    _by_step_n(P, 1, box)
+    o = _oracle(dims, 1, box)
+    assert np.abs(o.field("Ex").reshape(dims[::-1])[-1, -1]).max() > 0
+    _assert_equal(P, o, dims)
+    simFDTD("DeleteSimulation", P)
