@@ -876,6 +876,9 @@ __global__ void __launch_bounds__(kThreads<NG>, 1)
             p = f.cnt + cnt_e + c * f.ty_e + y;
         }
         if (!(ok = wait_rows(p, want, f.err))) break;
+        // what lanes 0 to 2 have acquired holds for the warp (a vote alone is
+        // not documented to order memory)
+        __syncwarp();
         if (!it.e && f.n_probes) {
           gather_probes(d, f.probe_z, f.probe_at, row0 + it.n, it.x0, it.x0 + G::BX, it.y0,
                         it.y0 + G::BY, it.kb, it.np, lane);
