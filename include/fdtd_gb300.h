@@ -497,9 +497,11 @@ int fdtd_estimate_device_bytes(int32_t I, int32_t J, int32_t K, int32_t pml, int
 int fdtd_division_plan(float dx, float out[4]);
 
 /* Evaluates that plan on the current GPU for every float bit pattern as a
- * numerator (2^32 inputs, about a second) and stores in *mismatches the
- * number whose quotient differs bitwise from the GPU's IEEE division a/dx
- * (no reference counterpart: a self-check). */
+ * numerator (2^32 inputs, about a second), also as the multi-step kernel
+ * takes it (several numerators together, on their own and beside a subnormal
+ * one), and stores in *mismatches the number whose quotient differs bitwise
+ * from the GPU's IEEE division a/dx (no reference counterpart: a
+ * self-check). */
 int fdtd_check_division(float dx, uint64_t *mismatches);
 
 /* Bounded-wait self-check on the current GPU: every pipeline wait of the

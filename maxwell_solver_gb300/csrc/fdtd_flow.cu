@@ -298,36 +298,38 @@ __device__ __forceinline__ void stp4(float2 *p, const P4 &r) {
 __device__ __noinline__ float2 div_pair(float2 a, float dx) {
   return make_float2(div_ieee(a.x, dx), div_ieee(a.y, dx));
 }
-// RN(a / dx) of small numerators (|a| < 1), y = RN(1/dx): v, the quotient of
+// RN(a / dx) of small numerators (|a| < lim = div_lim, from which a*2^100 would
+// leave the range of the corrected product), y = RN(1/dx): v, the quotient of
 // a*2^100, scaled back.  Where that rounds a second time (subnormal quotients)
 // the result differs from the right one only if v lies half way between two
 // subnormals without being exact; the remainder of v tells the side.  q: the
 // quotient of a*2^64, for the others.
-__device__ __forceinline__ float quot_small(float a, float q, float dx, float y) {
+__device__ __forceinline__ float quot_small(float a, float q, float dx, float y, float lim) {
   const float s = a * 0x1p100f, q0 = s * y;
   const float v = __fmaf_rn(__fmaf_rn(q0, dx, -s), -y, q0);
   const float r = __fmaf_rn(v, dx, -s);  // > 0: v is above the quotient
   const float w = v * 0x1p-100f, t = __fmaf_rn(w, -0x1p100f, v);
   const bool other = fabsf(t) == 0x1p-50f && r != 0.f && (r > 0.f) != (t > 0.f);
-  return fabsf(a) < 1.f ? w + (other ? copysignf(0x1p-149f, t) : copysignf(0.f, w)) : q * 0x1p-64f;
+  return fabsf(a) < lim ? w + (other ? copysignf(0x1p-149f, t) : copysignf(0.f, w)) : q * 0x1p-64f;
 }
-__device__ __noinline__ float2 quot_pair(float2 a, float2 q, float dx, float y) {
-  return make_float2(quot_small(a.x, q.x, dx, y), quot_small(a.y, q.y, dx, y));
+__device__ __noinline__ float2 quot_pair(float2 a, float2 q, float dx, float y, float lim) {
+  return make_float2(quot_small(a.x, q.x, dx, y, lim), quot_small(a.y, q.y, dx, y, lim));
 }
 
-// All eight quotients of a recurrence in one call.
+// All eight quotients of a recurrence in one call (lim < 0: divide).
 struct F8 {
   float2 v[4];
 };
-__device__ __noinline__ F8 quot_all(F8 a, F8 q, float dx, float y, bool divide) {
-  if (divide) {
+__device__ __noinline__ F8 quot_all(F8 a, F8 q, float dx, float y, float lim) {
+  if (lim < 0.f) {
 #pragma unroll
     for (int n = 0; n < 4; ++n) a.v[n] = div_pair(a.v[n], dx);
     return a;
   }
 #pragma unroll
   for (int n = 0; n < 4; ++n)
-    q.v[n] = make_float2(quot_small(a.v[n].x, q.v[n].x, dx, y), quot_small(a.v[n].y, q.v[n].y, dx, y));
+    q.v[n] = make_float2(quot_small(a.v[n].x, q.v[n].x, dx, y, lim),
+                         quot_small(a.v[n].y, q.v[n].y, dx, y, lim));
   return q;
 }
 
@@ -360,7 +362,7 @@ __device__ __forceinline__ P4 recur(const fdtd_dev &d, P4 ps, const Q4 &b, const
   float u = 0x1p-64f;
   if (least < __float_as_uint(d.div_lo2) * 2u - 1u || most >= d.div_hi * 0x1p-64f) {
     u = 1.f;
-    const bool divide = most >= d.div_hi * 0x1p-64f || d.div_lo > 0x1p-60f;
+    const bool divide = most >= d.div_hi * 0x1p-64f || d.div_lim == 0.f;
     if (ONE) {
       F8 x, z;
 #pragma unroll
@@ -368,13 +370,13 @@ __device__ __forceinline__ P4 recur(const fdtd_dev &d, P4 ps, const Q4 &b, const
         x.v[n] = a[n];
         z.v[n] = q[n];
       }
-      z = quot_all(x, z, d.dx, d.rdx, divide);
+      z = quot_all(x, z, d.dx, d.rdx, divide ? -1.f : d.div_lim);
 #pragma unroll
       for (int n = 0; n < 4; ++n) q[n] = z.v[n];
     } else {
 #pragma unroll
       for (int n = 0; n < 4; ++n)
-        q[n] = divide ? div_pair(a[n], d.dx) : quot_pair(a[n], q[n], d.dx, d.rdx);
+        q[n] = divide ? div_pair(a[n], d.dx) : quot_pair(a[n], q[n], d.dx, d.rdx, d.div_lim);
     }
   }
 #pragma unroll
@@ -385,6 +387,37 @@ __device__ __forceinline__ P4 recur(const fdtd_dev &d, P4 ps, const Q4 &b, const
   }
   return ps;
 }
+// Self-check of the recurrences' quotients over all float bit patterns, eight
+// of them at once, or seven beside a subnormal numerator (so that the special
+// path takes them): psi = -0 and b = c = 1 leave the bare quotient.
+template <bool ONE>
+__global__ void k_check_recurrence(const __grid_constant__ fdtd_dev d, int tiny,
+                                   unsigned long long *out) {
+  unsigned long long bad = 0;
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x, per = tiny ? 7 : 8;
+  for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t * per < 1ull << 32;
+       t += stride) {
+    Q4 a, b;
+    float v[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      v[e] = __uint_as_float(tiny && e == 7 ? 1u : (uint32_t)(t * per + e));
+      set(e < 4 ? a : b, e & 3, v[e]);
+    }
+    P4 ps;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) ps.c[e] = make_float2(-0.f, -0.f);
+    ps = recur<ONE>(d, ps, all4(1.f), all4(1.f), a, b);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const float got = e < 4 ? ps.c[e].x : ps.c[e - 4].y, want = v[e] / d.dx;
+      bad += __float_as_uint(got) != __float_as_uint(want) && !(got != got && want != want);
+    }
+  }
+  for (int o = 16; o > 0; o >>= 1) bad += __shfl_xor_sync(0xffffffffu, bad, o);
+  if ((threadIdx.x & 31) == 0 && bad) atomicAdd(out, bad);
+}
+
 // b, c of the four cells from i at their X slab positions (0 where the slab
 // function is negative, and the cell's bit in the result).
 template <class S>
@@ -1485,6 +1518,23 @@ int fdtdk_flow(const fdtd_dev *d, const fdtd_maps_flow *m, const fdtd_op *op, co
   if (d->hcoef_mode)
     return ob ? launch_coef<true, true>(d, m, op, w, s) : launch_coef<true, false>(d, m, op, w, s);
   return ob ? launch_coef<false, true>(d, m, op, w, s) : launch_coef<false, false>(d, m, op, w, s);
+}
+
+int fdtdk_check_recurrence(fdtd_div_plan p, unsigned long long *out, cudaStream_t s) {
+  fdtd_dev d;
+  memset(&d, 0, sizeof(d));
+  d.dx = p.dx;
+  d.rdx = p.rdx;
+  d.div_lo = p.lo;
+  d.div_hi = p.hi;
+  d.div_lo2 = p.lo2;
+  d.div_lim = p.lim;
+  for (int tiny = 0; tiny < 2; ++tiny) {
+    k_check_recurrence<true><<<152 * 8, 256, 0, s>>>(d, tiny, out);
+    k_check_recurrence<false><<<152 * 8, 256, 0, s>>>(d, tiny, out);
+  }
+  fdtdk_count_launches(4);
+  return (int)cudaGetLastError();
 }
 
 int64_t fdtdk_flow_counters(int32_t J, int32_t K) {

@@ -225,7 +225,7 @@ static float f32_from_bits(uint32_t u) {
 }
 
 static fdtd_div_plan div_plan_compute(float dx) {
-  fdtd_div_plan p = {dx, 1.0f / dx, INFINITY, 0.0f, INFINITY};
+  fdtd_div_plan p = {dx, 1.0f / dx, INFINITY, 0.0f, INFINITY, 0.0f};
   if (!isnormal(dx) || !(dx > 0.0f)) return p;
   const float y = (float)(1.0 / (double)dx);
   if (!isnormal(y)) return p;
@@ -266,6 +266,13 @@ static fdtd_div_plan div_plan_compute(float dx) {
   } else {
     p.lo2 = p.lo;
   }
+  /* scaling by 2^100 (quot_small in fdtd_flow.cu) takes every nonzero
+   * |a| < lim into [lo, hi): 2^-149 * 2^100 >= lo, and lim * 2^100 <= hi
+   * (lim is below 1 from dx = 2^-26 down); from lim on the scaling by 2^64 serves,
+   * so lim >= lo2.  Otherwise such numerators are divided (lim = 0). */
+  const float l3 = ldexpf(p.hi, -100);
+  p.lim = l3 < 1.0f ? l3 : 1.0f;
+  if (p.lo > 0x1p-60f || p.lim < p.lo2) p.lim = 0.0f;
   return p;
 }
 
@@ -784,6 +791,7 @@ static void fill_dev_struct(sim *s) {
     d->div_lo = dp.lo;
     d->div_hi = dp.hi;
     d->div_lo2 = dp.lo2;
+    d->div_lim = dp.lim;
   }
   memcpy(d->bE, s->bE, sizeof(d->bE));
   memcpy(d->cE, s->cE, sizeof(d->cE));
@@ -2519,6 +2527,7 @@ int fdtd_check_division(float dx, uint64_t *mismatches) {
   int rc = FDTD_OK;
   if (cudaMemset(d_bad, 0, sizeof(*d_bad)) != cudaSuccess ||
       fdtdk_check_division(p, 0, 1ull << 32, d_bad, 0) != 0 ||
+      fdtdk_check_recurrence(p, d_bad, 0) != 0 ||
       cudaMemcpy(&bad, d_bad, sizeof(bad), cudaMemcpyDeviceToHost) != cudaSuccess)
     rc = fail(FDTD_ERR_CUDA, "division check: %s", cudaGetErrorString(cudaGetLastError()));
   cudaFree(d_bad);

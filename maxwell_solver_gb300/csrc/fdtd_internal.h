@@ -54,8 +54,9 @@ typedef struct {
   float Chh, Che, dx;
   /* quotient x/dx: see fdtd_make_div_plan (rdx = RN(1/dx); the corrected
    * product is used for div_lo <= |x| < div_hi, and on x*2^64 for
-   * div_lo2 <= |x| < div_lo) */
-  float rdx, div_lo, div_hi, div_lo2;
+   * div_lo2 <= |x| < div_lo; the multi-step kernel may use it on x*2^100
+   * for |x| < div_lim) */
+  float rdx, div_lo, div_hi, div_lo2, div_lim;
   float bE[2 * FDTD_MAX_PML], cE[2 * FDTD_MAX_PML];
   float bH[2 * FDTD_MAX_PML], cH[2 * FDTD_MAX_PML];
   float *f[6];              /* Ex Ey Ez Hx Hy Hz, x-fastest IJK each */
@@ -401,20 +402,24 @@ int fdtdk_rasterize(const fdtd_dev *d, float *const sig[3], float *const eps[3],
 
 /* Plan for dividing by a fixed cell size (fdtd_host.c). */
 typedef struct {
-  float dx, rdx, lo, hi, lo2;
+  float dx, rdx, lo, hi, lo2, lim;
 } fdtd_div_plan;
 fdtd_div_plan fdtd_make_div_plan(float dx);
 /* Adds to *out (device) the number of float bit patterns in
  * [first, first + count) whose plan quotient differs bitwise from the IEEE
  * division on the GPU. */
+int fdtdk_check_division(fdtd_div_plan p, uint64_t first, uint64_t count,
+                         unsigned long long *out, cudaStream_t s);
+/* The same for the multi-step kernel's recurrences, over all patterns: each
+ * as they choose its path beside its neighbours, and each beside a subnormal
+ * numerator (any NaN for a NaN). */
+int fdtdk_check_recurrence(fdtd_div_plan p, unsigned long long *out, cudaStream_t s);
 /* Bounded-wait self-check (fdtd_tma.cu): out[0] = 1 when the wait gave up,
  * out[1] = global-timer ns it took; the production limit and the check's
  * (ns). */
 int fdtdk_check_wait(int arrive, long long out[2]);
 unsigned long long fdtdk_wait_ns(void);
 unsigned long long fdtdk_check_ns(void);
-int fdtdk_check_division(fdtd_div_plan p, uint64_t first, uint64_t count,
-                         unsigned long long *out, cudaStream_t s);
 
 #ifdef __cplusplus
 }
