@@ -2292,10 +2292,11 @@ static int flow_usable(sim *s, int32_t mode, const fdtd_current *cur) {
   return fdtd_flow_ok(&s->dev, &o);
 }
 
-/* n steps from `first` on the handle's stream, zc planes an item; on at most
- * `blocks` SMs (0: all), errors reported in *err (device). */
+/* n steps from `first` on the handle's stream, at most `most` a launch, zc
+ * planes an item; on at most `blocks` SMs (0: all), errors reported in *err
+ * (device). */
 static int run_flow(sim *s, int32_t first, int32_t count, int32_t mode, const fdtd_current *cur,
-                    int32_t zc, int32_t blocks, int32_t *err) {
+                    int32_t most, int32_t zc, int32_t blocks, int32_t *err) {
   fdtd_flow w;
   memset(&w, 0, sizeof(w));
   if (s->flow_counted != zc) {
@@ -2317,10 +2318,6 @@ static int run_flow(sim *s, int32_t first, int32_t count, int32_t mode, const fd
   }
   fdtd_op o;
   step_op_e(s, &o, mode, cur);
-  /* A launch lasts some 10 ms at most, so that other streams' work gets its
-   * turn; its tickets then fit their 32-bit counter many times over. */
-  const int64_t cs = (int64_t)1 << (blocks ? 31 : 29);
-  const int32_t most = s->cells < cs / 8 ? (int32_t)(cs / s->cells) : 8;
   for (int32_t done = 0; done < count; done += w.n_steps) {
     w.n_steps = count - done < most ? count - done : most;
     w.first = first + done;
@@ -2329,6 +2326,13 @@ static int run_flow(sim *s, int32_t first, int32_t count, int32_t mode, const fd
     s->flow_base += (uint32_t)w.n_steps;
   }
   return FDTD_OK;
+}
+
+/* Steps of a launch that take 2^shift cell-steps or less (8 steps at least):
+ * far fewer tickets than their 32-bit counter holds. */
+static int32_t flow_steps(const sim *s, int shift) {
+  const int64_t cs = (int64_t)1 << shift;
+  return s->cells < cs / 8 ? (int32_t)(cs / s->cells) : 8;
 }
 
 /* Steps first..first+count-1 as GRAPH_CHUNK-step graph replays and single
@@ -2342,8 +2346,15 @@ static int run_steps(sim *s, int32_t first, int32_t count, int32_t mode,
   /* Multi-step launches unless FDTD_FUSED=1 asked for the fused pairs: they
    * are faster than either other way at every size measured (24^3 to 512^3). */
   const int forced = s->fused_forced && fused_usable(s, mode, cur);
-  if (!forced && flow_usable(s, mode, cur))
-    return run_flow(s, first, count, mode, cur, s->flow_zc, 0, s->d_err);
+  if (!forced && flow_usable(s, mode, cur)) {
+    /* Launches of some milliseconds, so that other streams' work gets its turn:
+     * 2^29 cell-steps (6 ms at the rate of large grids), and 256 steps, since a
+     * step takes 9 us or more however small the grid (a launch's start and end
+     * cost 5 us: 64^3, 2048 steps in one call: 12.54 us a step as one launch,
+     * 12.57 as eight). */
+    const int32_t most = flow_steps(s, 29);
+    return run_flow(s, first, count, mode, cur, most < 256 ? most : 256, s->flow_zc, 0, s->d_err);
+  }
   if (count >= 2 && fused_usable(s, mode, cur)) return run_fused(s, first, count, mode);
   if (count >= GRAPH_CHUNK) {
     const int cm = use_cur ? cur->mode : 0;
@@ -3268,8 +3279,11 @@ static int batch_flow(batch *b, const int32_t *steps) {
     const double at_all = (double)s->cells * sms / blocks;
     int32_t zc = at_all < 350000 ? 1 : at_all < 1100000 ? 2 : at_all < FLOW_BIG ? 4 : 8;
     if (zc > s->K) zc = s->K;
-    rc = run_flow(s, m->first + m->done, steps[sh[g].g], m->mode, m->has_cur ? &m->cur : NULL, zc,
-                  blocks, b->d_err);
+    /* Up to a second on four SMs: the streams share a few hardware queues, where
+     * a member's next launch, waiting for the one before, holds up other
+     * members' first ones. */
+    rc = run_flow(s, m->first + m->done, steps[sh[g].g], m->mode, m->has_cur ? &m->cur : NULL,
+                  flow_steps(s, 31), zc, blocks, b->d_err);
   }
   free(sh);
   /* the batch's stream follows every member: after all launches, since the
