@@ -175,7 +175,10 @@ typedef struct sim {
   uint32_t *d_flow;
   uint32_t flow_base;
   int32_t flow_counted;
-  int32_t flow_tile, flow_zc;
+  int32_t flow_tile;
+  cudaEvent_t busy_ev;  /* after the last steps issued */
+  int busy_issuing;     /* ... which are being issued (g_busy_lock) */
+  int device;
   int32_t *d_pz, *d_pat, n_pat;     /* n_pat -1: a probe position it cannot serve */
 } sim;
 
@@ -365,6 +368,52 @@ static cudaError_t pool_alloc(void **p, size_t bytes, cudaStream_t st) {
 }
 
 
+/* The handles whose steps may be unfinished (at most MAX_BUSY are known). */
+#define MAX_BUSY 152
+static pthread_mutex_t g_busy_lock = PTHREAD_MUTEX_INITIALIZER;
+static sim *g_busy[MAX_BUSY];
+static int g_n_busy = 0;
+
+/* The handle is about to issue steps; returns how many handles of its device
+ * have some, this one included.  busy_issued follows. */
+static int busy_enter(sim *s) {
+  int n = 1, kept = 0, known = 0;
+  pthread_mutex_lock(&g_busy_lock);
+  for (int a = 0; a < g_n_busy; ++a) {
+    sim *t = g_busy[a];
+    if (t == s) {
+      known = 1;
+    } else if (t->busy_issuing || cudaEventQuery(t->busy_ev) == cudaErrorNotReady) {
+      n += t->device == s->device;
+    } else {
+      continue; /* finished */
+    }
+    g_busy[kept++] = t;
+  }
+  if (kept > known) cudaGetLastError(); /* the queries' "not ready" */
+  if (!known && kept < MAX_BUSY) g_busy[kept++] = s;
+  g_n_busy = kept;
+  s->busy_issuing = 1;
+  pthread_mutex_unlock(&g_busy_lock);
+  return n;
+}
+static int busy_issued(sim *s) {
+  const cudaError_t e = cudaEventRecord(s->busy_ev, s->stream);
+  pthread_mutex_lock(&g_busy_lock);
+  s->busy_issuing = 0;
+  pthread_mutex_unlock(&g_busy_lock);
+  CU(e);
+  return FDTD_OK;
+}
+/* The handle goes away. */
+static void busy_leave(sim *s) {
+  pthread_mutex_lock(&g_busy_lock);
+  for (int a = 0; a < g_n_busy; ++a)
+    if (g_busy[a] == s) g_busy[a--] = g_busy[--g_n_busy];
+  pthread_mutex_unlock(&g_busy_lock);
+  if (s->busy_ev) cudaEventDestroy(s->busy_ev);
+}
+
 int fdtd_create(fdtd_handle *out) {
   if (!out) return fail(FDTD_ERR_INVALID_ARG, "null output handle");
   sim *s = (sim *)calloc(1, sizeof(sim));
@@ -382,6 +431,8 @@ int fdtd_create(fdtd_handle *out) {
     return fail(FDTD_ERR_CUDA, "cudaStreamCreate: %s", cudaGetErrorString(e));
   }
   for (int i = 0; i < MAX_EVENTS; ++i) cudaEventCreate(&s->ev[i]);
+  cudaEventCreateWithFlags(&s->busy_ev, cudaEventDisableTiming);
+  cudaGetDevice(&s->device);
   pthread_mutex_lock(&g_reg_lock);
   int slot = -1;
   for (int i = 0; i < MAX_SIMS; ++i)
@@ -392,6 +443,7 @@ int fdtd_create(fdtd_handle *out) {
   if (slot < 0) {
     pthread_mutex_unlock(&g_reg_lock);
     for (int i = 0; i < MAX_EVENTS; ++i) cudaEventDestroy(s->ev[i]);
+    cudaEventDestroy(s->busy_ev);
     cudaStreamDestroy(s->stream);
     free(s);
     return fail(FDTD_ERR_OOM, "too many live simulations");
@@ -415,6 +467,7 @@ int fdtd_destroy(fdtd_handle h) {
   g_sims[slot - 1] = NULL;
   pthread_mutex_unlock(&g_reg_lock);
   cudaStreamSynchronize(s->stream);
+  busy_leave(s);
   if (s->gexec) cudaGraphExecDestroy(s->gexec);
   if (s->gexec_f) cudaGraphExecDestroy(s->gexec_f);
   dfree(s->d_psib_pool);
@@ -1215,21 +1268,32 @@ static int fused_mode(void) {
   return -1;
 }
 
-/* The multi-step kernel's counters, its item geometry and its probe lists by
- * z-plane. */
 #define FLOW_BIG 4000000 /* cells */
+/* z-planes of an item on `blocks` of the GPU's SMs: a half-step should have an
+ * item or more for each of the 456 groups (3 on each of 152 SMs), then as many
+ * planes as that leaves, since an item's waits, first loads and face pass cost
+ * as much as several planes.  Measured from rest (us a step at 1/2/4/8 planes
+ * an item; mode 0, then mode 5): 64^3 11.1/14.0/21.4/- and 26.5/29.7/34.6/-;
+ * 80^3 13/16/22/36 and 34/30/34/48; 112^3 30/25/28/38 and 70/54/41/49; 144^3
+ * 61/49/48/58 and 112/91/73/72; 192^3 -/102/96/97 and -/153/123/117; modes 1-4
+ * lie between.  16 planes are slower everywhere. */
+static int32_t flow_height(const sim *s, int32_t blocks, int32_t sms) {
+  const double at_all = (double)s->cells * sms / blocks;
+  const int32_t zc = at_all < 350000 ? 1 : at_all < 1100000 ? 2 : at_all < FLOW_BIG ? 4 : 8;
+  return zc < s->K ? zc : s->K;
+}
+
+static int sm_count(void) {
+  int sms = 0, dev = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms < 1 ? 1 : sms;
+}
+
+/* The multi-step kernel's counters, its tile and its probe lists by z-plane. */
 static int flow_setup(sim *s) {
   s->flow_counted = 0;
-  /* Item height: a half-step should have an item or more for each of the
-   * 456 groups (3 on each of 152 SMs), then as many planes as that leaves,
-   * since an item's waits, first loads and face pass cost as much as several
-   * planes.  Measured from rest (us a step at 1/2/4/8 planes an item; mode 0,
-   * then mode 5): 64^3 11.1/14.0/21.4/- and 26.5/29.7/34.6/-; 80^3 13/16/22/36
-   * and 34/30/34/48; 112^3 30/25/28/38 and 70/54/41/49; 144^3 61/49/48/58 and
-   * 112/91/73/72; 192^3 -/102/96/97 and -/153/123/117; modes 1-4 lie between.
-   * 16 planes are slower everywhere.
-   *
-   * From 4 million cells on the fields (24 B a cell) and the psi pairs outgrow
+  /* From 4 million cells on the fields (24 B a cell) and the psi pairs outgrow
    * the L2 cache, and the pairs are fetched ahead (without / with, 8 planes:
    * 128^3 54/55 in mode 5, 160^3 80/74, 256^3 238/225, 320^3 439/418).
    *
@@ -1239,8 +1303,6 @@ static int flow_setup(sim *s) {
    * 168/159, 512x512x448 1381/1354). */
   const int big = s->cells >= FLOW_BIG;
   s->flow_tile = big && s->I >= 320 ? 0 : 1;
-  s->flow_zc = s->cells < 350000 ? 1 : s->cells < 1100000 ? 2 : big ? 8 : 4;
-  if (s->flow_zc > s->K) s->flow_zc = s->K;
   /* one allocation: the probes by plane, each plane's first, the counters */
   const int K = s->K, probes = s->init_ant && s->num_ant > 0 ? s->num_ant : 0;
   const size_t lists = probes ? 4 * (size_t)probes + (((size_t)K + 1 + 3) & ~(size_t)3) : 0;
@@ -2335,10 +2397,11 @@ static int32_t flow_steps(const sim *s, int shift) {
   return s->cells < cs / 8 ? (int32_t)(cs / s->cells) : 8;
 }
 
-/* Steps first..first+count-1 as GRAPH_CHUNK-step graph replays and single
- * steps (the arguments already checked). */
-static int run_steps(sim *s, int32_t first, int32_t count, int32_t mode,
-                     const fdtd_current *cur) {
+/* Steps first..first+count-1 as multi-step launches, or as GRAPH_CHUNK-step
+ * graph replays and single steps (the arguments already checked); n: the
+ * handles that have steps on the device, this one included. */
+static int issue_steps(sim *s, int32_t first, int32_t count, int32_t mode,
+                       const fdtd_current *cur, int n) {
   int rc;
   const int use_cur = cur && cur->mode >= 1 && cur->mode <= 3;
   const int probes = s->dev.num_ant > 0;
@@ -2346,14 +2409,27 @@ static int run_steps(sim *s, int32_t first, int32_t count, int32_t mode,
   /* Multi-step launches unless FDTD_FUSED=1 asked for the fused pairs: they
    * are faster than either other way at every size measured (24^3 to 512^3). */
   const int forced = s->fused_forced && fused_usable(s, mode, cur);
-  if (!forced && flow_usable(s, mode, cur)) {
+  /* Not mode 5 on grids of one-plane items beside other handles: 64^3, us for a
+   * step of all, separate kernels / launches on parts of the GPU: 2 handles
+   * 29.8/32.7, 4 40.0/51.0, 8 70.9/71.6; 8 of 40^3 32.4/49.6. */
+  const int beside = n > 1 && mode == FDTD_MODE_OBLIQUE && flow_height(s, 1, 1) == 1;
+  if (!forced && !beside && flow_usable(s, mode, cur)) {
     /* Launches of some milliseconds, so that other streams' work gets its turn:
      * 2^29 cell-steps (6 ms at the rate of large grids), and 256 steps, since a
      * step takes 9 us or more however small the grid (a launch's start and end
      * cost 5 us: 64^3, 2048 steps in one call: 12.54 us a step as one launch,
      * 12.57 as eight). */
     const int32_t most = flow_steps(s, 29);
-    return run_flow(s, first, count, mode, cur, most < 256 ? most : 256, s->flow_zc, 0, s->d_err);
+    /* Handles that run at the same time (in one thread or several) take an equal
+     * part of the SMs each: launches on all of them would follow one another,
+     * and a small grid's step is a chain of waits that leaves the SMs idle.
+     * Eight handles, us for a step of all, separate kernels / launches on all SMs
+     * / on parts, 32 steps a call: mode 0 40^3 28/78/23, 64^3 63/82/40, 96^3
+     * 209/123/118; mode 5 96^3 227/272/155, 144^3 535/530/457. */
+    const int sms = sm_count();
+    const int32_t part = sms / n > 4 ? sms / n : 4;
+    return run_flow(s, first, count, mode, cur, most < 256 ? most : 256,
+                    flow_height(s, part, sms), n > 1 ? part : 0, s->d_err);
   }
   if (count >= 2 && fused_usable(s, mode, cur)) return run_fused(s, first, count, mode);
   if (count >= GRAPH_CHUNK) {
@@ -2397,6 +2473,13 @@ static int run_steps(sim *s, int32_t first, int32_t count, int32_t mode,
   for (; done < count; ++done)
     if ((rc = step_ops(s, first + done, 0, mode, cur))) return rc;
   return FDTD_OK;
+}
+
+static int run_steps(sim *s, int32_t first, int32_t count, int32_t mode,
+                     const fdtd_current *cur) {
+  const int rc = issue_steps(s, first, count, mode, cur, busy_enter(s));
+  const int rc2 = busy_issued(s);
+  return rc ? rc : rc2;
 }
 
 int fdtd_profile_steps(fdtd_handle h, int32_t first, int32_t count, int32_t mode,
@@ -3171,13 +3254,6 @@ static int batch_rebuild_(batch *b) {
   return FDTD_OK;
 }
 
-static int sm_count(void) {
-  int sms = 0, dev = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  return sms < 1 ? 1 : sms;
-}
-
 /* The active members, and how they run. */
 static int batch_list(batch *b) {
   if (b->n > b->act_cap) {
@@ -3275,10 +3351,7 @@ static int batch_flow(batch *b, const int32_t *steps) {
     sim *s = lookup(m->h);
     const double share = ceil(sh[g].work / hi);
     const int32_t blocks = share < 1 ? 1 : (share > sms ? sms : (int32_t)share);
-    /* items as in flow_setup's rule, for this member's part of the SMs */
-    const double at_all = (double)s->cells * sms / blocks;
-    int32_t zc = at_all < 350000 ? 1 : at_all < 1100000 ? 2 : at_all < FLOW_BIG ? 4 : 8;
-    if (zc > s->K) zc = s->K;
+    const int32_t zc = flow_height(s, blocks, sms);
     /* Up to a second on four SMs: the streams share a few hardware queues, where
      * a member's next launch, waiting for the one before, holds up other
      * members' first ones. */
