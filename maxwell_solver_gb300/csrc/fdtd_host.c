@@ -1276,10 +1276,26 @@ static int fused_mode(void) {
  * an item; mode 0, then mode 5): 64^3 11.1/14.0/21.4/- and 26.5/29.7/34.6/-;
  * 80^3 13/16/22/36 and 34/30/34/48; 112^3 30/25/28/38 and 70/54/41/49; 144^3
  * 61/49/48/58 and 112/91/73/72; 192^3 -/102/96/97 and -/153/123/117; modes 1-4
- * lie between.  16 planes are slower everywhere. */
-static int32_t flow_height(const sim *s, int32_t blocks, int32_t sms) {
+ * lie between.  16 planes are slower everywhere.
+ * In mode 5 an item's face pass costs by the face planes it meets, so narrow
+ * and long grids want one plane (faces within the planes) or tall items sooner;
+ * the line lies by the number of one-plane items (by cells alone / so, separate
+ * kernels): 80^3 31/27, 35; 100^3 50/40, 43; 40x500x40 49/36, 45; 64x64x250
+ * 47/38, 42; 48x100x180 53/42, 43; 40x40x1500 120/96, 101; 150^3 81/75, 92; where
+ * the former line is kept 96^3 35, 131x117x109 51, 120x60x120 39 (38). */
+static int64_t flow_items(const sim *s) {
+  return (int64_t)((s->I + 31) / 32) * ((s->J + 15) / 16) * s->K;
+}
+static int32_t flow_height(const sim *s, int32_t mode, int32_t blocks, int32_t sms) {
   const double at_all = (double)s->cells * sms / blocks;
-  const int32_t zc = at_all < 350000 ? 1 : at_all < 1100000 ? 2 : at_all < FLOW_BIG ? 4 : 8;
+  int32_t zc = at_all < 350000 ? 1 : at_all < 1100000 ? 2 : at_all < FLOW_BIG ? 4 : 8;
+  if (mode == FDTD_MODE_OBLIQUE && blocks == sms && zc != 1 && s->cells < FLOW_BIG) {
+    const int64_t n = flow_items(s);
+    zc = n <= 1600 || (n <= 3100 && s->K <= 80)    ? 1
+         : n <= 1950                               ? 2
+         : n <= 3700 || (n <= 5000 && s->K < 200) ? 4
+                                                   : 8;
+  }
   return zc < s->K ? zc : s->K;
 }
 
@@ -2397,6 +2413,23 @@ static int32_t flow_steps(const sim *s, int shift) {
   return s->cells < cs / 8 ? (int32_t)(cs / s->cells) : 8;
 }
 
+/* Where multi-step launches are slower than the separate kernels, all in mode 5:
+ * - small grids beside other handles (64^3, us for a step of all, separate
+ *   kernels / launches on parts of the GPU: 2 handles 29.8/32.7, 4 40.0/51.0, 8
+ *   70.9/71.6; 8 of 40^3 32.4/49.6);
+ * - long grids of a small section, where every item meets faces of two axes and
+ *   there are more items than groups (40x40x500 46/51, 34x34x600 48/57, 60x60x200
+ *   36/40, 40x60x260 41/46, 34x34x1000 67/71; beyond the line 50x50x600 61/60,
+ *   40x40x1500 101/96, 64x64x250 42/38; per-cell H coefficients favour the
+ *   launches: 40x40x500 50/54, 60x60x200 39/44, but 56x56x300 47/43, 24x24x2000
+ *   84/73). */
+static int flow_slower(const sim *s, int32_t mode, int n) {
+  if (mode != FDTD_MODE_OBLIQUE) return 0;
+  if (n > 1 && s->cells < 350000) return 1;
+  return (int64_t)s->I * s->J <= 3600 && s->K > 80 && flow_items(s) >= 1500 &&
+         s->cells < (s->hcoef_mode ? 900000 : 1400000);
+}
+
 /* Steps first..first+count-1 as multi-step launches, or as GRAPH_CHUNK-step
  * graph replays and single steps (the arguments already checked); n: the
  * handles that have steps on the device, this one included. */
@@ -2409,11 +2442,7 @@ static int issue_steps(sim *s, int32_t first, int32_t count, int32_t mode,
   /* Multi-step launches unless FDTD_FUSED=1 asked for the fused pairs: they
    * are faster than either other way at every size measured (24^3 to 512^3). */
   const int forced = s->fused_forced && fused_usable(s, mode, cur);
-  /* Not mode 5 on grids of one-plane items beside other handles: 64^3, us for a
-   * step of all, separate kernels / launches on parts of the GPU: 2 handles
-   * 29.8/32.7, 4 40.0/51.0, 8 70.9/71.6; 8 of 40^3 32.4/49.6. */
-  const int beside = n > 1 && mode == FDTD_MODE_OBLIQUE && flow_height(s, 1, 1) == 1;
-  if (!forced && !beside && flow_usable(s, mode, cur)) {
+  if (!forced && !flow_slower(s, mode, n) && flow_usable(s, mode, cur)) {
     /* Launches of some milliseconds, so that other streams' work gets its turn:
      * 2^29 cell-steps (6 ms at the rate of large grids), and 256 steps, since a
      * step takes 9 us or more however small the grid (a launch's start and end
@@ -2429,7 +2458,7 @@ static int issue_steps(sim *s, int32_t first, int32_t count, int32_t mode,
     const int sms = sm_count();
     const int32_t part = sms / n > 4 ? sms / n : 4;
     return run_flow(s, first, count, mode, cur, most < 256 ? most : 256,
-                    flow_height(s, part, sms), n > 1 ? part : 0, s->d_err);
+                    flow_height(s, mode, part, sms), n > 1 ? part : 0, s->d_err);
   }
   if (count >= 2 && fused_usable(s, mode, cur)) return run_fused(s, first, count, mode);
   if (count >= GRAPH_CHUNK) {
@@ -3351,7 +3380,7 @@ static int batch_flow(batch *b, const int32_t *steps) {
     sim *s = lookup(m->h);
     const double share = ceil(sh[g].work / hi);
     const int32_t blocks = share < 1 ? 1 : (share > sms ? sms : (int32_t)share);
-    const int32_t zc = flow_height(s, blocks, sms);
+    const int32_t zc = flow_height(s, m->mode, blocks, sms);
     /* Up to a second on four SMs: the streams share a few hardware queues, where
      * a member's next launch, waiting for the one before, holds up other
      * members' first ones. */

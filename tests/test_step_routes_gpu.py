@@ -1,0 +1,78 @@
+"""Whole steps on every route a StepN call may take, against the FP32 oracle,
+bit for bit (every route does the same roundings): the item heights of mode 5,
+and the separate half-step kernels where multi-step launches are not taken."""
+import math
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+FIELDS = ("Ex", "Ey", "Ez", "Hx", "Hy", "Hz")
+
+
+def _run_equal(dims, pml, inset, steps, mode, probes=None, calls=(1, 9)):
+    """StepN in calls of 1, 9 and the remaining steps; returns the launches of
+    the last call."""
+    import oracle
+    from maxwell_solver_gb300 import launch_count, simFDTD
+
+    rng = np.random.default_rng(sum(dims))
+    dx = 1e-3
+    fr = np.float32([20e9, dx, 0.9 * dx / (math.sqrt(3) * 299792458.0)])
+    td = np.int32([steps, *dims, 0 if probes is None else len(probes)])
+    pulse = np.sin(0.4 * np.arange(steps) + 0.3).astype(np.float32)
+    eps = (1 + rng.integers(0, 4, dims)).ravel(order="F").astype(np.float32)
+    P = simFDTD("CreateSimulation")
+    o = oracle.OracleSim("f32")
+    simFDTD("SetParams", P, np.float64([pml, inset, 3, 1, 0.08, 1, 0.8, 0]))
+    o.set_params(pml=pml, tfsf_width=inset)
+    simFDTD("SetConst", P, fr, td)
+    o.set_const(fr, td)
+    if probes is not None:
+        simFDTD("SetAntennaLocations", P, np.asfortranarray(np.int32(probes)))
+        o.set_antenna_locations(np.asfortranarray(np.int32(probes)))
+    simFDTD("UpdateMaterial", P, np.int32(5), eps)
+    o.update_material(5, eps)
+    simFDTD("ReadySimulation", P)
+    o.ready_simulation()
+    if mode == 5:
+        simFDTD("SetIncidence", P, np.float64([0.9, -0.6, 1.2]))
+        o.set_incidence(0.9, -0.6, 1.2)
+    if mode:
+        simFDTD("Init1D", P, np.float32(1), pulse)
+        o.init_1d(1.0, pulse)
+    at = 0
+    for n in (*calls, steps - sum(calls)):
+        before = launch_count()
+        simFDTD("StepN", P, np.int32([at, n, mode]))
+        at += n
+    launches = launch_count() - before
+    for n in range(steps):
+        o.step(n, mode)
+    for f, field in enumerate(FIELDS, 1):
+        got = simFDTD("OutputVis", P, np.uint32(np.prod(dims)), np.int32(f))
+        np.testing.assert_array_equal(got, o.field(field), err_msg=field)
+    if probes is not None:
+        rec = simFDTD("OutputProbes", P, np.uint32(steps * len(probes) * 6))
+        np.testing.assert_array_equal(rec, o.array("probes"))
+    if mode:
+        assert max(np.abs(o.field(f)).max() for f in FIELDS) > 0
+    simFDTD("DeleteSimulation", P)
+    return launches
+
+
+@pytest.mark.parametrize("dims, pml, steps", [
+    ((45, 130, 79), 6, 40),     # one plane an item: few of them
+    ((41, 301, 80), 6, 30),     # one plane: K <= 80
+    ((95, 96, 97), 6, 40),      # two planes
+    ((47, 99, 181), 6, 30),     # four planes
+    ((40, 1003, 41), 6, 24),    # eight planes: many items
+    ((65, 66, 313), 6, 24),     # eight planes: long
+])
+def test_item_heights_of_mode_5(dims, pml, steps):
+    assert _run_equal(dims, pml, pml + 2, steps, 5) == 1
+
+
+def test_long_grids_of_a_small_section_in_mode_5_take_the_separate_kernels():
+    assert _run_equal((38, 41, 262), 6, 8, 60, 5) > 50
