@@ -3283,8 +3283,8 @@ static int batch_rebuild_(batch *b) {
   return FDTD_OK;
 }
 
-/* The active members, and how they run. */
-static int batch_list(batch *b) {
+/* The active members, and how they run (to_end: this call is to finish them). */
+static int batch_list(batch *b, int to_end) {
   if (b->n > b->act_cap) {
     int *a = (int *)realloc(b->act, (size_t)b->n * sizeof(int));
     if (!a) return fail(FDTD_ERR_OOM, "out of host memory");
@@ -3299,16 +3299,21 @@ static int batch_list(batch *b) {
     if (!s) return fail(FDTD_ERR_INVALID_HANDLE, "a batch member was deleted");
     b->act[b->n_act++] = i;
   }
-  /* On their own SMs the members need four each: with fewer, rounding the shares
-   * to whole SMs and the rate of one SM on a small grid cost more than the
-   * launches.  300 steps of members of 32..128 cells a side, mode 5, separate
-   * kernels / multi-step launches (ms): 4 members 29.6/17.1, 8 48.7/36.5, 16
-   * 53.3/40.2, 24 94.7/91.0, 32 105/101, 40 120/121, 48 149/169; 32..56 a side:
-   * 24 28.2/22.5, 40 41.7/35.7; 100..160, mode 1, 60 steps: 32 67.3/62.9. */
-  b->flow = b->n_act * 4 <= sm_count();
+  /* On their own SMs the members need at least four each, with the plane wave's
+   * faces more: with fewer, rounding the shares to whole SMs and the rate of one
+   * SM on a small grid cost more than the launches.  Steps of all members
+   * together (us, separate kernels / multi-step launches, 32 steps a call): mode
+   * 5, 32..128 cells a side: 16 members 231/207, 20 237/240, 24 329/343, 32
+   * 439/524; mode 1, 100..160: 20 876/779, 24 1046/1013, 28 1066/1080, 38
+   * 1503/1605; mode 0, 48..140: 16 329/286, 28 504/470, 38 667/644.  To the end
+   * in one call, members of 150..300 steps (ms): mode 5 20 43.5/38.8, 28
+   * 72.8/66.5, 32 81.5/88.1; mode 1 24 202/202. */
+  double need = 0;
+  b->flow = 1;
   for (int g = 0; g < b->n_act && b->flow; ++g) {
     const bmember *m = &b->m[b->act[g]];
-    b->flow = flow_usable(lookup(m->h), m->mode, m->has_cur ? &m->cur : NULL);
+    need += m->mode == 0 ? 4 : m->mode != FDTD_MODE_OBLIQUE ? 6 : to_end ? 5.4 : 7.5;
+    b->flow = need <= sm_count() && flow_usable(lookup(m->h), m->mode, m->has_cur ? &m->cur : NULL);
   }
   b->mirrored = 0;
   b->dirty = 0;
@@ -3481,7 +3486,7 @@ static int batch_advance(batch *b, int32_t max_steps, int to_end, int32_t *activ
   if (active_left) *active_left = left;
   if (!left || max_steps <= 0) return FDTD_OK;
   if (b->dirty) {
-    if ((rc = batch_list(b))) return rc;
+    if ((rc = batch_list(b, to_end))) return rc;
     /* new members: their own queued work must be on the device first */
     for (int g = 0; g < b->n_act; ++g)
       if ((rc = flush(lookup(b->m[b->act[g]].h)))) return rc;

@@ -76,3 +76,46 @@ def test_item_heights_of_mode_5(dims, pml, steps):
 
 def test_long_grids_of_a_small_section_in_mode_5_take_the_separate_kernels():
     assert _run_equal((38, 41, 262), 6, 8, 60, 5) > 50
+
+
+@pytest.mark.parametrize("to_end", [False, True])
+def test_batch_of_24_in_mode_5(to_end):
+    """Stepped together they run as separate kernels, to the end in one call as
+    multi-step launches; each ends as alone."""
+    from maxwell_solver_gb300 import launch_count, simFDTD
+    from maxwell_solver_gb300.batch import Batch
+
+    dims = [(26 + g % 7, 27 + g % 5, 26 + g % 9) for g in range(24)]
+    steps = [60 + g % 4 for g in range(24)]
+
+    def ready(d):
+        P = simFDTD("CreateSimulation")
+        simFDTD("SetParams", P, np.float64([5, 7, 3, 1, 0.08, 1, 0.8, 0]))
+        simFDTD("SetConst", P, np.float32([20e9, 1e-3, 1.7e-12]), np.int32([70, *d, 0]))
+        simFDTD("ReadySimulation", P)
+        simFDTD("SetIncidence", P, np.float64([0.9, -0.6, 1.2]))
+        simFDTD("Init1D", P, np.float32(1), np.sin(0.4 * np.arange(70)).astype(np.float32))
+        return P
+
+    Ps = [ready(d) for d in dims]
+    with Batch() as b:
+        for P, n in zip(Ps, steps):
+            b.add(P, 0, n, 5)
+        before = launch_count()
+        if to_end:
+            b.run()
+            # one each, and 12 steps that measure the separate kernels' z-run
+            assert launch_count() - before <= 24 + 12 * 6
+        else:
+            b.step(32)
+            assert launch_count() - before > 24 + 12 * 6
+            b.run()
+    for P, d, n in zip(Ps, dims, steps):
+        Q = ready(d)
+        simFDTD("StepN", Q, np.int32([0, n, 5]))
+        for f in range(1, 7):
+            cells = np.uint32(np.prod(d))
+            np.testing.assert_array_equal(simFDTD("OutputVis", P, cells, np.int32(f)),
+                                          simFDTD("OutputVis", Q, cells, np.int32(f)))
+        simFDTD("DeleteSimulation", P)
+        simFDTD("DeleteSimulation", Q)
