@@ -158,8 +158,8 @@ struct Flow {
   int tx_h, ty_h, tx_e, ty_e;
   int tiles, per_half;      // tickets per chunk and per half-step
   Div by_step, by_tiles, by_tx;
-  const int32_t *probe_z;   // [K+1] first entry of each plane
-  const int4 *probe_at;     // {probe, i, j, 0} by plane
+  const int32_t *probe_first;  // [tiles * K + 1] first entry of each tile's planes
+  const int2 *probe_at;     // {probe, cell} in that order
   int n_probes;             // probe entries (0: none)
 };
 
@@ -788,23 +788,23 @@ __device__ __forceinline__ Item decode(const Flow &f, int K, int w) {
   return it;
 }
 
-// The probes in an H item's cells: E and H at the start of the step (nothing
-// of it has been overwritten yet), by the producer warp.
-__device__ __noinline__ void gather_probes(const fdtd_dev &d, const int32_t *pz, const int4 *pat,
-                                           int row, int x0, int x1, int y0, int y1, int kb,
-                                           int np, int lane) {
-  const int a = pz[kb], b = pz[kb + np];
+// The probes in an H item's cells (a list per tile and plane, `first` at the
+// item's): E and H at the start of the step (nothing of it has been overwritten
+// yet), by the producer warp.  With one list per plane, which every tile's item
+// looked through, a dense plane of probes cost more than the separate gather (us
+// a step, separate kernels / so / with a list per tile: 64^3 and 2304 probes in a
+// plane 35/49/19, 128^3 and 8100 85/108/37, 200^3 and 10000 207/216/108).
+__device__ __noinline__ void gather_probes(const fdtd_dev &d, const int32_t *first,
+                                           const int2 *pat, int row, int np, int lane) {
+  const int a = first[0], b = first[np];
   if (row >= d.T) return;
 #pragma unroll 1
   for (int t = a + lane; t < b; t += 32) {
-    const int4 e = pat[t];
-    const int i = min(e.y, d.I - 2), j = min(e.z, d.J - 2);
-    if (i < x0 || i >= x1 || j < y0 || j >= y1) continue;
-    const int64_t id = d.probe_idx[e.x];
+    const int2 e = pat[t];
     float *o = d.probes + ((int64_t)row * d.num_ant + e.x) * 6;
     float v[6];
 #pragma unroll
-    for (int c = 0; c < 6; ++c) v[c] = __ldcg(d.f[c] + id);
+    for (int c = 0; c < 6; ++c) v[c] = __ldcg(d.f[c] + e.y);
 #pragma unroll
     for (int c = 0; c < 6; ++c) o[c] = v[c];
   }
@@ -913,8 +913,8 @@ __global__ void __launch_bounds__(kThreads<NG>, 1)
         // not documented to order memory)
         __syncwarp();
         if (!it.e && f.n_probes) {
-          gather_probes(d, f.probe_z, f.probe_at, row0 + it.n, it.x0, it.x0 + G::BX, it.y0,
-                        it.y0 + G::BY, it.kb, it.np, lane);
+          gather_probes(d, f.probe_first + (it.ty * f.tx_e + it.x0 / G::BX) * d.K + it.kb,
+                        f.probe_at, row0 + it.n, it.np, lane);
           __syncwarp();
         }
         if (lane == 0) {
@@ -1452,8 +1452,8 @@ int launch(const fdtd_dev *d, const fdtd_maps_flow *m, const fdtd_op *op, const 
   const long long tickets = 2ll * f.per_half * w->n_steps;
   if (tickets > (1ll << 30) || tickets < 1) return (int)cudaErrorInvalidValue;
   f.n_tickets = (int)tickets;
-  f.probe_z = w->probe_z;
-  f.probe_at = reinterpret_cast<const int4 *>(w->probe_at);
+  f.probe_first = w->probe_first;
+  f.probe_at = reinterpret_cast<const int2 *>(w->probe_at);
   f.n_probes = w->n_probes;
   const long long want = (2ll * f.tiles * f.nch_e + NG - 1) / NG;  // a step's items
   int blocks = want < cached ? (int)want : cached;

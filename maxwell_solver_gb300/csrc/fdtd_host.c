@@ -179,7 +179,7 @@ typedef struct sim {
   cudaEvent_t busy_ev;  /* after the last steps issued */
   int busy_issuing;     /* ... which are being issued (g_busy_lock) */
   int device;
-  int32_t *d_pz, *d_pat, n_pat;     /* n_pat -1: a probe position it cannot serve */
+  int32_t *d_pfirst, *d_pat, n_pat; /* n_pat -1: a probe position it cannot serve */
 } sim;
 
 /* ------------------------------------------------------------ registry */
@@ -1306,7 +1306,7 @@ static int sm_count(void) {
   return sms < 1 ? 1 : sms;
 }
 
-/* The multi-step kernel's counters, its tile and its probe lists by z-plane. */
+/* The multi-step kernel's counters, its tile and its probe lists. */
 static int flow_setup(sim *s) {
   s->flow_counted = 0;
   /* From 4 million cells on the fields (24 B a cell) and the psi pairs outgrow
@@ -1319,9 +1319,14 @@ static int flow_setup(sim *s) {
    * 168/159, 512x512x448 1381/1354). */
   const int big = s->cells >= FLOW_BIG;
   s->flow_tile = big && s->I >= 320 ? 0 : 1;
-  /* one allocation: the probes by plane, each plane's first, the counters */
+  /* one allocation: the probes by item column (a tile's z-planes; tiles as the
+   * queue numbers them) and plane, the first of each plane, the counters */
   const int K = s->K, probes = s->init_ant && s->num_ant > 0 ? s->num_ant : 0;
-  const size_t lists = probes ? 4 * (size_t)probes + (((size_t)K + 1 + 3) & ~(size_t)3) : 0;
+  const int bx = s->flow_tile ? FDTD_BTILE_X : FDTD_TILE_X;
+  const int by = s->flow_tile ? FDTD_BTILE_Y : FDTD_TILE_Y;
+  const int tx = (s->I + bx - 1) / bx, ty = (s->J + by - 1) / by;
+  const size_t planes = (size_t)tx * ty * K, at = 2 * (size_t)probes;
+  const size_t lists = probes ? at + ((planes + 1 + 3) & ~(size_t)3) : 0;
   const size_t counters = (size_t)fdtdk_flow_counters(s->J, K);
   int rc = dalloc(s, (void **)&s->d_flow_mem, (lists + counters) * sizeof(int32_t));
   if (rc) return rc;
@@ -1329,41 +1334,38 @@ static int flow_setup(sim *s) {
   s->n_pat = 0;
   if (!probes) return FDTD_OK;
   s->d_pat = s->d_flow_mem;
-  s->d_pz = s->d_flow_mem + 4 * (size_t)probes;
+  s->d_pfirst = s->d_flow_mem + at;
   /* kept until the handle goes: the copy below may still read it */
   free(s->h_flow);
   s->h_flow = (int32_t *)calloc(lists, sizeof(int32_t));
-  int32_t *at = (int32_t *)calloc((size_t)K, sizeof(int32_t));
-  if (!s->h_flow || !at) {
-    free(at);
-    return fail(FDTD_ERR_OOM, "out of host memory");
-  }
-  int32_t *pat = s->h_flow, *pz = s->h_flow + 4 * (size_t)probes;
+  if (!s->h_flow) return fail(FDTD_ERR_OOM, "out of host memory");
+  int32_t *pat = s->h_flow, *first = s->h_flow + at;
   /* a probe belongs to the H item whose cells hold it, the last plane, row
-   * and column to the ones before them */
+   * and column to the ones before them; count, sum up, then fill from the ends
+   * back, which leaves each plane's first */
   for (int pass = 0; pass < 2; ++pass) {
-    for (int a = 0; a < s->num_ant; ++a) {
+    for (int a = 0; a < probes; ++a) {
       const int64_t id = s->h_probe_idx[a];
       if (id < 0) continue; /* outside: its record stays zero */
       const int k = (int)(id / s->plane), j = (int)(id % s->plane / s->Ip);
       const int i = (int)(id % s->Ip), kk = k < K - 2 ? k : K - 2;
+      const int ii = i < s->I - 2 ? i : s->I - 2, jj = j < s->J - 2 ? j : s->J - 2;
+      int32_t *at_plane = first + ((size_t)(jj / by * tx + ii / bx) * K + kk);
       if (pass == 0) {
-        pz[kk + 1] += 1;
+        *at_plane += 1;
         /* the last row of the last plane: E there is not among what the H
          * item waits for */
         if (k == K - 1 && j == s->J - 1) s->n_pat = -1;
       } else {
-        int32_t *e = pat + 4 * (size_t)(pz[kk] + at[kk]++);
+        int32_t *e = pat + 2 * (size_t)--*at_plane;
         e[0] = a;
-        e[1] = i;
-        e[2] = j;
+        e[1] = (int32_t)id; /* fdtd_flow_ok: fits */
       }
     }
     if (pass == 0)
-      for (int k = 0; k < K; ++k) pz[k + 1] += pz[k];
+      for (size_t k = 0; k < planes; ++k) first[k + 1] += first[k];
   }
-  free(at);
-  if (s->n_pat == 0) s->n_pat = s->num_ant;
+  if (s->n_pat == 0) s->n_pat = probes;
   CU(cudaMemcpyAsync(s->d_flow_mem, s->h_flow, lists * sizeof(int32_t), cudaMemcpyHostToDevice,
                      s->stream));
   return FDTD_OK;
@@ -2390,7 +2392,7 @@ static int run_flow(sim *s, int32_t first, int32_t count, int32_t mode, const fd
   w.blocks = blocks;
   w.err = err;
   if (s->dev.num_ant > 0) {
-    w.probe_z = s->d_pz;
+    w.probe_first = s->d_pfirst;
     w.probe_at = s->d_pat;
     w.n_probes = s->n_pat;
   }
@@ -2619,8 +2621,10 @@ int fdtd_estimate_device_bytes(int32_t I, int32_t J, int32_t K, int32_t pml, int
   b += cells * 2 + (uint64_t)MAX_MATERIALS * 6 * 4; /* material ids + table */
   b += (uint64_t)HASH_CAP * (8 + 8 + 4) + 16 + 4;  /* indexing scratch, error word */
   b += 2 * psi * 4;                                /* psi pairs */
-  b += (uint64_t)fdtdk_flow_counters(J, K) * 4 +
-       ((uint64_t)K + 4 + 4 * (uint64_t)num_ant) * 4; /* multi-step counters, probe lists */
+  b += (uint64_t)fdtdk_flow_counters(J, K) * 4; /* multi-step counters, probe lists */
+  if (num_ant > 0)
+    b += 8 * (uint64_t)num_ant +
+         4 * ((uint64_t)((I + 31) / 32) * ((J + 7) / 8) * K + 4); /* (of the smaller tile sides) */
   if (fused_mode() == 1 || (fused_mode() < 0 && tune_enabled() &&
                               (int64_t)cells >= TUNE_MIN_CELLS))
     b += 6 * cells * 4 + psi * 4;                  /* the fused step's second buffer

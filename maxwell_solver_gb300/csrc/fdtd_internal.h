@@ -274,8 +274,8 @@ typedef struct {
   int32_t blocks;           /* SMs to use at most (0: all) */
   int32_t *err;             /* device error word */
   int32_t ahead;            /* tile 1: psi pairs come to L2 a plane ahead (tile 0: always) */
-  const int32_t *probe_z;   /* [K+1] first probe entry of each z-plane */
-  const int32_t *probe_at;  /* {probe, i, j, 0} by plane */
+  const int32_t *probe_first; /* [tiles * K + 1] first probe entry of each tile's planes */
+  const int32_t *probe_at;  /* {probe, cell} in that order */
   int32_t n_probes;
 } fdtd_flow;
 /* Counters a grid needs at any tile geometry and item height. */

@@ -119,3 +119,23 @@ def test_batch_of_24_in_mode_5(to_end):
                                           simFDTD("OutputVis", Q, cells, np.int32(f)))
         simFDTD("DeleteSimulation", P)
         simFDTD("DeleteSimulation", Q)
+
+
+def _dense(dims, pml):
+    """Probe positions (relative to the CPML) on an inner z-plane and on the
+    last planes of the three axes, without the edge j = J-1, k = K-1."""
+    I, J, K = (d - pml for d in dims)
+    at = [(i, j, K // 2) for i in range(0, I, 2) for j in range(0, J)]
+    at += [(I - 1, j, k) for j in range(0, J - 1, 3) for k in range(0, K, 2)]
+    at += [(i, J - 1, k) for i in range(0, I, 5) for k in range(0, K - 1, 3)]
+    at += [(i, j, K - 1) for i in range(0, I, 4) for j in range(0, J - 1, 5)]
+    return at
+
+
+@pytest.mark.parametrize("dims, pml, steps, mode", [
+    ((45, 50, 41), 5, 24, 3),      # one plane an item
+    ((97, 81, 67), 6, 16, 0),      # two planes
+    ((331, 113, 109), 8, 12, 5),   # eight planes, tiles of 64 x 8
+])
+def test_dense_probes(dims, pml, steps, mode):
+    assert _run_equal(dims, pml, pml + 2, steps, mode, _dense(dims, pml)) == 1
