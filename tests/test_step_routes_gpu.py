@@ -139,3 +139,14 @@ def _dense(dims, pml):
 ])
 def test_dense_probes(dims, pml, steps, mode):
     assert _run_equal(dims, pml, pml + 2, steps, mode, _dense(dims, pml)) == 1
+
+
+@pytest.mark.parametrize("tile", ["0", "1", "2"])
+@pytest.mark.parametrize("mode", [0, 1, 3, 5])
+def test_separate_kernels_with_a_probe_on_the_outer_edge(mode, tile, monkeypatch):
+    """A probe at j = J-1, k = K-1: the steps run as separate half-step kernels
+    in every tile geometry, 32 of them as a graph replay."""
+    monkeypatch.setenv("FDTD_TILE", tile)
+    dims, pml = (70, 53, 42), 5
+    corner = [(20, dims[1] - 1 - pml, dims[2] - 1 - pml), (30, 20, 11)]
+    assert _run_equal(dims, pml, pml + 2, 60, mode, corner) > 50
