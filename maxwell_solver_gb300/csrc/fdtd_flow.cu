@@ -298,38 +298,36 @@ __device__ __forceinline__ void stp4(float2 *p, const P4 &r) {
 __device__ __noinline__ float2 div_pair(float2 a, float dx) {
   return make_float2(div_ieee(a.x, dx), div_ieee(a.y, dx));
 }
-// RN(a / dx) of small numerators (|a| < lim = div_lim, from which a*2^100 would
-// leave the range of the corrected product), y = RN(1/dx): v, the quotient of
-// a*2^100, scaled back.  Where that rounds a second time (subnormal quotients)
+// RN(a / dx) of small numerators (|a| < 1, where div_small), y = RN(1/dx): v, the
+// quotient of a*2^100, scaled back.  Where that rounds a second time (subnormal quotients)
 // the result differs from the right one only if v lies half way between two
 // subnormals without being exact; the remainder of v tells the side.  q: the
 // quotient of a*2^64, for the others.
-__device__ __forceinline__ float quot_small(float a, float q, float dx, float y, float lim) {
+__device__ __forceinline__ float quot_small(float a, float q, float dx, float y) {
   const float s = a * 0x1p100f, q0 = s * y;
   const float v = __fmaf_rn(__fmaf_rn(q0, dx, -s), -y, q0);
   const float r = __fmaf_rn(v, dx, -s);  // > 0: v is above the quotient
   const float w = v * 0x1p-100f, t = __fmaf_rn(w, -0x1p100f, v);
   const bool other = fabsf(t) == 0x1p-50f && r != 0.f && (r > 0.f) != (t > 0.f);
-  return fabsf(a) < lim ? w + (other ? copysignf(0x1p-149f, t) : copysignf(0.f, w)) : q * 0x1p-64f;
+  return fabsf(a) < 1.f ? w + (other ? copysignf(0x1p-149f, t) : copysignf(0.f, w)) : q * 0x1p-64f;
 }
-__device__ __noinline__ float2 quot_pair(float2 a, float2 q, float dx, float y, float lim) {
-  return make_float2(quot_small(a.x, q.x, dx, y, lim), quot_small(a.y, q.y, dx, y, lim));
+__device__ __noinline__ float2 quot_pair(float2 a, float2 q, float dx, float y) {
+  return make_float2(quot_small(a.x, q.x, dx, y), quot_small(a.y, q.y, dx, y));
 }
 
-// All eight quotients of a recurrence in one call (lim < 0: divide).
+// All eight quotients of a recurrence in one call.
 struct F8 {
   float2 v[4];
 };
-__device__ __noinline__ F8 quot_all(F8 a, F8 q, float dx, float y, float lim) {
-  if (lim < 0.f) {
+__device__ __noinline__ F8 quot_all(F8 a, F8 q, float dx, float y, bool divide) {
+  if (divide) {
 #pragma unroll
     for (int n = 0; n < 4; ++n) a.v[n] = div_pair(a.v[n], dx);
     return a;
   }
 #pragma unroll
   for (int n = 0; n < 4; ++n)
-    q.v[n] = make_float2(quot_small(a.v[n].x, q.v[n].x, dx, y, lim),
-                         quot_small(a.v[n].y, q.v[n].y, dx, y, lim));
+    q.v[n] = make_float2(quot_small(a.v[n].x, q.v[n].x, dx, y), quot_small(a.v[n].y, q.v[n].y, dx, y));
   return q;
 }
 
@@ -362,7 +360,7 @@ __device__ __forceinline__ P4 recur(const fdtd_dev &d, P4 ps, const Q4 &b, const
   float u = 0x1p-64f;
   if (least < __float_as_uint(d.div_lo2) * 2u - 1u || most >= d.div_hi * 0x1p-64f) {
     u = 1.f;
-    const bool divide = most >= d.div_hi * 0x1p-64f || d.div_lim == 0.f;
+    const bool divide = most >= d.div_hi * 0x1p-64f || !d.div_small;
     if (ONE) {
       F8 x, z;
 #pragma unroll
@@ -370,13 +368,13 @@ __device__ __forceinline__ P4 recur(const fdtd_dev &d, P4 ps, const Q4 &b, const
         x.v[n] = a[n];
         z.v[n] = q[n];
       }
-      z = quot_all(x, z, d.dx, d.rdx, divide ? -1.f : d.div_lim);
+      z = quot_all(x, z, d.dx, d.rdx, divide);
 #pragma unroll
       for (int n = 0; n < 4; ++n) q[n] = z.v[n];
     } else {
 #pragma unroll
       for (int n = 0; n < 4; ++n)
-        q[n] = divide ? div_pair(a[n], d.dx) : quot_pair(a[n], q[n], d.dx, d.rdx, d.div_lim);
+        q[n] = divide ? div_pair(a[n], d.dx) : quot_pair(a[n], q[n], d.dx, d.rdx);
     }
   }
 #pragma unroll
@@ -1528,7 +1526,7 @@ int fdtdk_check_recurrence(fdtd_div_plan p, unsigned long long *out, cudaStream_
   d.div_lo = p.lo;
   d.div_hi = p.hi;
   d.div_lo2 = p.lo2;
-  d.div_lim = p.lim;
+  d.div_small = p.small;
   for (int tiny = 0; tiny < 2; ++tiny) {
     k_check_recurrence<true><<<152 * 8, 256, 0, s>>>(d, tiny, out);
     k_check_recurrence<false><<<152 * 8, 256, 0, s>>>(d, tiny, out);

@@ -228,7 +228,7 @@ static float f32_from_bits(uint32_t u) {
 }
 
 static fdtd_div_plan div_plan_compute(float dx) {
-  fdtd_div_plan p = {dx, 1.0f / dx, INFINITY, 0.0f, INFINITY, 0.0f};
+  fdtd_div_plan p = {dx, 1.0f / dx, INFINITY, 0.0f, INFINITY, 0};
   if (!isnormal(dx) || !(dx > 0.0f)) return p;
   const float y = (float)(1.0 / (double)dx);
   if (!isnormal(y)) return p;
@@ -269,13 +269,13 @@ static fdtd_div_plan div_plan_compute(float dx) {
   } else {
     p.lo2 = p.lo;
   }
-  /* scaling by 2^100 (quot_small in fdtd_flow.cu) takes every nonzero
-   * |a| < lim into [lo, hi): 2^-149 * 2^100 >= lo, and lim * 2^100 <= hi
-   * (lim is below 1 from dx = 2^-26 down); from lim on the scaling by 2^64 serves,
-   * so lim >= lo2.  Otherwise such numerators are divided (lim = 0). */
-  const float l3 = ldexpf(p.hi, -100);
-  p.lim = l3 < 1.0f ? l3 : 1.0f;
-  if (p.lo > 0x1p-60f || p.lim < p.lo2) p.lim = 0.0f;
+  /* scaling by 2^100 (quot_small in fdtd_flow.cu) takes every nonzero |a| < 1
+   * to lo or above (2^-149 * 2^100 >= lo) and keeps a*2^100*y finite (y < 2^28;
+   * dx > 3.7e-9).  Otherwise such numerators are divided: on nanometre grids
+   * that costs time while a wave's front is in the CPML, where passing the
+   * numerator up to which the scaling holds to quot_small cost every grid: mode
+   * 5 4 % on 131x117x109, the others 1 %. */
+  p.small = p.lo <= 0x1p-60f && y < 0x1p28f;
   return p;
 }
 
@@ -844,7 +844,7 @@ static void fill_dev_struct(sim *s) {
     d->div_lo = dp.lo;
     d->div_hi = dp.hi;
     d->div_lo2 = dp.lo2;
-    d->div_lim = dp.lim;
+    d->div_small = dp.small;
   }
   memcpy(d->bE, s->bE, sizeof(d->bE));
   memcpy(d->cE, s->cE, sizeof(d->cE));

@@ -54,9 +54,9 @@ typedef struct {
   float Chh, Che, dx;
   /* quotient x/dx: see fdtd_make_div_plan (rdx = RN(1/dx); the corrected
    * product is used for div_lo <= |x| < div_hi, and on x*2^64 for
-   * div_lo2 <= |x| < div_lo; the multi-step kernel may use it on x*2^100
-   * for |x| < div_lim) */
-  float rdx, div_lo, div_hi, div_lo2, div_lim;
+   * div_lo2 <= |x| < div_lo, and if div_small on x*2^100 for |x| < 1) */
+  float rdx, div_lo, div_hi, div_lo2;
+  int32_t div_small;
   float bE[2 * FDTD_MAX_PML], cE[2 * FDTD_MAX_PML];
   float bH[2 * FDTD_MAX_PML], cH[2 * FDTD_MAX_PML];
   float *f[6];              /* Ex Ey Ez Hx Hy Hz, x-fastest IJK each */
@@ -402,7 +402,8 @@ int fdtdk_rasterize(const fdtd_dev *d, float *const sig[3], float *const eps[3],
 
 /* Plan for dividing by a fixed cell size (fdtd_host.c). */
 typedef struct {
-  float dx, rdx, lo, hi, lo2, lim;
+  float dx, rdx, lo, hi, lo2;
+  int32_t small;
 } fdtd_div_plan;
 fdtd_div_plan fdtd_make_div_plan(float dx);
 /* Adds to *out (device) the number of float bit patterns in
