@@ -12,15 +12,15 @@
  * Order and waits.  Tickets are taken from a global counter in order: step by
  * step, the H items by z-chunk and tile, then the E items.  Item (half, step,
  * chunk c, tile row ty, tile column) waits for
- *   H of step n: E of step n-1 in the rows (c, ty), (c, ty+1), (c+1, ty);
- *   E of step n: H of step n   in the rows (c, ty), (c, ty-1), (c-1, ty),
+ *   H of step n: E of step n-1 in the rows (c, ty), (c, ty+1), (c+1, ty), (c+1, ty+1);
+ *   E of step n: H of step n   in the rows (c, ty), (c, ty-1), (c-1, ty), (c-1, ty-1),
  * every tile column of a row counted together.  Those rows hold what the item
- * reads, and every reader of what it overwrites (a tile's halo also brings
- * cells that nothing uses, and those are not waited for).  H has no cells at
- * j = J-1 and k = K-1: where a row of E items holds just these (J-1 and K-1
- * multiples of the tile's height and of the item's planes), none of the three
- * H rows exists, and the items wait for their own row of step n-1, whose cells
- * they go on from.  All of these are earlier in the
+ * reads, and every reader of what it overwrites.  The fourth holds no cell that
+ * the item uses, but H has no cells at j = J-1 and k = K-1: where a row of E
+ * items holds just these (J-1 and K-1 multiples of the tile's height and of the
+ * item's planes), the fourth is the only one there is, and orders such an item
+ * after itself of step n-1 (as a wait of its own it cost 1 % on 64^3 and
+ * 131x117x109).  All of these are earlier in the
  * order, so the earliest unfinished item can always run and no ticket waits
  * for a block that is not running.  A row's counter counts finished tiles
  * and is never reset within a launch (`base` steps were counted before
@@ -893,21 +893,17 @@ __global__ void __launch_bounds__(kThreads<NG>, 1)
         uint32_t want;
         if (it.e) {
           want = (uint32_t)f.tx_h * (f.base + it.n + 1);
-          const int c = it.c - (lane == 2), y = it.ty - (lane == 1);
-          if (lane < 3 && c >= 0 && y >= 0 && c < f.nch_h && y < f.ty_h)
+          const int c = it.c - (lane >> 1), y = it.ty - (lane & 1);
+          if (lane < 4 && c >= 0 && y >= 0 && c < f.nch_h && y < f.ty_h)
             p = f.cnt + c * f.ty_h + y;
-          if (lane == 0 && it.c >= f.nch_h && it.ty >= f.ty_h) {  // the edge beyond all H cells
-            want = (uint32_t)f.tx_e * (f.base + it.n);
-            p = f.cnt + cnt_e + it.c * f.ty_e + it.ty;
-          }
         } else {
           want = (uint32_t)f.tx_e * (f.base + it.n);
-          const int c = it.c + (lane == 2), y = it.ty + (lane == 1);
-          if (lane < 3 && it.n > 0 && c < f.nch_e && y < f.ty_e)
+          const int c = it.c + (lane >> 1), y = it.ty + (lane & 1);
+          if (lane < 4 && it.n > 0 && c < f.nch_e && y < f.ty_e)
             p = f.cnt + cnt_e + c * f.ty_e + y;
         }
         if (!(ok = wait_rows(p, want, f.err))) break;
-        // what lanes 0 to 2 have acquired holds for the warp (a vote alone is
+        // what lanes 0 to 3 have acquired holds for the warp (a vote alone is
         // not documented to order memory)
         __syncwarp();
         if (!it.e && f.n_probes) {
