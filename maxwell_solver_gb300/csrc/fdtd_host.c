@@ -1518,29 +1518,40 @@ typedef struct {
   int64_t psi_floats, probe_floats;
 } ckpt_header;
 
-/* Copies the psi pairs between the device arrays' padded rows and the
- * image's dense ones (dense: device memory, psi_floats values). */
-static int ckpt_psi(sim *s, float *dense, int to_dense) {
+/* Copies the psi pairs between the device arrays' padded rows and the image's
+ * dense ones: by way of dense rows in device memory, or, where none is left for
+ * them, straight from or into the image (a row is a few dozen bytes on the X
+ * axis: slow, but it needs no memory). */
+static int ckpt_psi(sim *s, float *dense, float *image, int save) {
   const size_t pair = 2 * sizeof(float);
   const int p = s->p;
-  float *at = dense;
+  float *at = dense ? dense : image;
   for (int a = 0; a < FDTD_NUM_PSI; ++a) {
     const int x = a == PSI_EX || a == PSI_HX, y = a == PSI_EY || a == PSI_HY;
-    const size_t rows = x ? (size_t)s->J * s->K : (y ? (size_t)2 * p * s->K : (size_t)2 * p * s->J);
+    const size_t rows = x ? (size_t)s->J * s->K : (size_t)2 * p * (y ? s->K : s->J);
     const size_t pitch = (size_t)(x ? s->pxp : s->Ip) * pair;
     const size_t width = (size_t)(x ? 2 * p : s->I) * pair;
     for (int part = 0; part < (x ? 2 : 1); ++part) { /* X: the low and the high slab */
       unsigned char *pad = (unsigned char *)s->d_psi[a] + (part ? (size_t)(p + s->pxo) * pair : 0);
       unsigned char *den = (unsigned char *)at + (part ? (size_t)p * pair : 0);
       const size_t w = x ? (size_t)p * pair : width;
-      if (to_dense)
-        CU(cudaMemcpy2DAsync(den, width, pad, pitch, w, rows, cudaMemcpyDeviceToDevice, s->stream));
-      else
-        CU(cudaMemcpy2DAsync(pad, pitch, den, width, w, rows, cudaMemcpyDeviceToDevice, s->stream));
+      const enum cudaMemcpyKind kind = dense ? cudaMemcpyDeviceToDevice
+                                       : save  ? cudaMemcpyDeviceToHost
+                                               : cudaMemcpyHostToDevice;
+      if (save) CU(cudaMemcpy2DAsync(den, width, pad, pitch, w, rows, kind, s->stream));
+      else CU(cudaMemcpy2DAsync(pad, pitch, den, width, w, rows, kind, s->stream));
     }
     at += rows * (width / sizeof(float));
   }
   return FDTD_OK;
+}
+
+/* The scratch for that (NULL: no memory left). */
+static float *ckpt_scratch(sim *s, size_t bytes) {
+  float *dense = NULL;
+  if (injected_alloc_failure()) return NULL;
+  if (pool_alloc((void **)&dense, bytes, s->stream) != cudaSuccess) cudaGetLastError();
+  return dense;
 }
 
 static void ckpt_describe(const sim *s, ckpt_header *hd) {
@@ -1591,11 +1602,10 @@ int fdtd_checkpoint_save(fdtd_handle h, void *buf, size_t n) {
   for (int a = 0; a < 6; ++a, o += fb)
     CU(cudaMemcpyAsync(o, s->d_f[a], fb, cudaMemcpyDeviceToHost, s->stream));
   const size_t pb = (size_t)hd.psi_floats * sizeof(float);
-  float *dense = NULL;
-  CU(pool_alloc((void **)&dense, pb, s->stream));
-  rc = ckpt_psi(s, dense, 1);
+  float *dense = ckpt_scratch(s, pb);
+  rc = ckpt_psi(s, dense, (float *)o, 1);
   const cudaError_t pe =
-      rc ? cudaSuccess : cudaMemcpyAsync(o, dense, pb, cudaMemcpyDeviceToHost, s->stream);
+      rc || !dense ? cudaSuccess : cudaMemcpyAsync(o, dense, pb, cudaMemcpyDeviceToHost, s->stream);
   dfree(dense);
   if (rc) return rc;
   CU(pe);
@@ -1630,10 +1640,10 @@ int fdtd_checkpoint_load(fdtd_handle h, const void *buf, size_t n) {
   for (int a = 0; a < 6; ++a, o += fb)
     CU(cudaMemcpyAsync(s->d_f[a], o, fb, cudaMemcpyHostToDevice, s->stream));
   const size_t pb = (size_t)want.psi_floats * sizeof(float);
-  float *dense = NULL;
-  CU(pool_alloc((void **)&dense, pb, s->stream));
-  const cudaError_t pe = cudaMemcpyAsync(dense, o, pb, cudaMemcpyHostToDevice, s->stream);
-  rc = pe == cudaSuccess ? ckpt_psi(s, dense, 0) : FDTD_OK;
+  float *dense = ckpt_scratch(s, pb);
+  const cudaError_t pe =
+      dense ? cudaMemcpyAsync(dense, o, pb, cudaMemcpyHostToDevice, s->stream) : cudaSuccess;
+  rc = pe == cudaSuccess ? ckpt_psi(s, dense, (float *)o, 0) : FDTD_OK;
   dfree(dense);
   CU(pe);
   if (rc) return rc;
