@@ -155,6 +155,13 @@ def ncu_traffic(workload: str) -> dict:
         return {}
 
 
+def multi_traffic(tr, steps, launches):
+    """DRAM bytes of an average multi-step launch: the profile has them per
+    step (None where it has none)."""
+    per_step = tr.get("step_dram_bytes_multi")
+    return per_step * steps // launches if per_step else None
+
+
 # ----------------------------------------------------------------- CPU arm
 
 def cpu_oracle_rate(w, target_s: float, max_steps: int, warmup: int = 3):
@@ -339,7 +346,7 @@ def run_ours(args, ranks):
                      "avg_launch_ms": round(ms.value / launches, 5),
                      "achieved": round(gbs(s_bytes, step_ms), 1),
                      "frac": round(gbs(s_bytes, step_ms) / peak, 4),
-                     "traffic": tr.get("k_flow_bytes_per_launch")}
+                     "traffic": multi_traffic(tr, K, launches)}
         dom = "S"
     d = kern[dom]
     step_comp = (kern["F"]["alg_bytes_per_cell"] if fused and not multi else
