@@ -150,3 +150,17 @@ def test_separate_kernels_with_a_probe_on_the_outer_edge(mode, tile, monkeypatch
     dims, pml = (70, 53, 42), 5
     corner = [(20, dims[1] - 1 - pml, dims[2] - 1 - pml), (30, 20, 11)]
     assert _run_equal(dims, pml, pml + 2, 60, mode, corner) > 50
+
+
+def test_separate_kernels_with_compacted_x():
+    """The same with the compacted CPML X kernels (FDTD_XC=1, read once per
+    process: in a child process)."""
+    import os
+    import subprocess
+    import sys
+
+    r = subprocess.run([sys.executable, "-m", "pytest", "-q", "-x", "-m", "gpu", "-k",
+                        "probe_on_the_outer_edge", os.path.abspath(__file__)],
+                       env=dict(os.environ, FDTD_XC="1"), capture_output=True, text=True,
+                       timeout=300)
+    assert r.returncode == 0, r.stdout[-3000:] + r.stderr[-2000:]
