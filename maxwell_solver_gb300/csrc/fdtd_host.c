@@ -2021,8 +2021,11 @@ static void set_current(const sim *s, fdtd_op *o, int32_t mode, const int32_t bo
 }
 
 /* A half-step of a whole step: curl, CPML and the step's TF/SF and current
- * source (if any). */
-static int whole_half(const fdtd_op *o) {
+ * source (if any).  Not mode 5 with the source on a face, which no kernel takes:
+ * held back, such a step would report its error up to GRAPH_CHUNK steps late. */
+static int whole_half(const sim *s, const fdtd_op *o) {
+  if (o->tfsf_mode == FDTD_MODE_OBLIQUE && o->cur_mode && !fdtd_tfsf_faces_clear(&s->dev, o))
+    return 0;
   return o->curl && o->pml && !o->step_from_dev;
 }
 
@@ -2060,13 +2063,13 @@ static int retire(sim *s) {
   s->pend.active = 0;
   const fdtd_op *o = &s->pend.op;
   int rc;
-  if (s->pend.h == 1 && s->gather_pending && !s->held_h && whole_half(o)) {
+  if (s->pend.h == 1 && s->gather_pending && !s->held_h && whole_half(s, o)) {
     s->held_h = 1;
     s->held_op = *o;
     s->gather_pending = 0;
     return FDTD_OK;
   }
-  if (s->pend.h == 0 && s->held_h && whole_half(o) && o->tfsf_mode == s->held_op.tfsf_mode &&
+  if (s->pend.h == 0 && s->held_h && whole_half(s, o) && o->tfsf_mode == s->held_op.tfsf_mode &&
       (!o->tfsf_mode || o->step == s->held_op.step)) {
     const int32_t n = o->cur_mode ? o->step : s->held_op.step, m = o->tfsf_mode;
     fdtd_current cur;

@@ -164,3 +164,29 @@ def test_separate_kernels_with_compacted_x():
                        env=dict(os.environ, FDTD_XC="1"), capture_output=True, text=True,
                        timeout=300)
     assert r.returncode == 0, r.stdout[-3000:] + r.stderr[-2000:]
+
+
+def test_a_source_on_a_face_in_mode_5_is_refused_at_its_step():
+    """Per-op calls: the next step's first call reports it, not a later one."""
+    from maxwell_solver_gb300 import SimFDTDError, simFDTD
+
+    dims, pml, steps = (40, 36, 34), 5, 8
+    P = simFDTD("CreateSimulation")
+    simFDTD("SetParams", P, np.float64([pml, pml + 3, 3, 1, 0.08, 1, 0.8, 0]))
+    simFDTD("SetConst", P, np.float32([20e9, 1e-3, 1.7e-12]), np.int32([steps, *dims, 0]))
+    pulse = np.sin(0.4 * np.arange(steps)).astype(np.float32)
+    simFDTD("SetSource", P, pulse)
+    simFDTD("ReadySimulation", P)
+    simFDTD("SetIncidence", P, np.float64([0.9, -0.6, 1.2]))
+    simFDTD("Init1D", P, np.float32(1), pulse)
+    tm = np.int32([0, 5])
+    simFDTD("UpdateH_All", P)
+    simFDTD("UpdateH_PlaneWave", P, tm)
+    simFDTD("UpdateH_PML", P)
+    simFDTD("UpdateE_All", P)
+    simFDTD("UpdateE_PlaneWave", P, tm)
+    simFDTD("UpdateE_PML", P)
+    simFDTD("AddCurrents", P, np.int32([0, 1]), np.int32([pml + 3, pml + 3, 12, 14, 12, 14]))
+    with pytest.raises(SimFDTDError):
+        simFDTD("UpdateH_All", P)
+    simFDTD("DeleteSimulation", P)
