@@ -207,9 +207,11 @@ typedef struct {
 /* Runs steps first..first+count-1 of the reference step order
  * (highfrequency.m:85-91, plus AddCurrents as in GICsimulation.m:119-124
  * when cur != NULL and cur->mode != 0), many steps per launch; steps that
- * cannot run so take two fused half-step kernels each, the loop captured in a
- * CUDA graph.  tfsf_mode 0 skips the plane-wave corrections.  Bitwise
- * identical to issuing the per-op calls. */
+ * cannot run so, or faster otherwise, take two fused half-step kernels each, the
+ * loop captured in a CUDA graph.  tfsf_mode 0 skips the plane-wave corrections;
+ * cells of the current's box outside the grid take nothing.  Identical to issuing
+ * the per-op calls (zeros of E on the grid's x faces may differ in sign).
+ * Handles whose steps are on the device at the same time share the GPU. */
 int fdtd_step_n(fdtd_handle h, int32_t first, int32_t count, int32_t tfsf_mode,
                 const fdtd_current *cur);
 
@@ -252,7 +254,9 @@ int fdtd_get_table(fdtd_handle h, int32_t which, float *out, size_t n);
  * Load it into a handle set up the same way (SetParams, SetConst, media,
  * probes, ReadySimulation, Init1D) and stepping continues exactly as the
  * saved handle would have (steps are numbered by the caller, as always).
- * A different set-up is rejected with FDTD_ERR_INVALID_ARG. */
+ * A different set-up is rejected with FDTD_ERR_INVALID_ARG.  The psi arrays are
+ * copied by way of device memory of their size where there is some, otherwise
+ * more slowly without. */
 int fdtd_checkpoint_size(fdtd_handle h, size_t *bytes);
 int fdtd_checkpoint_save(fdtd_handle h, void *buf, size_t n);
 int fdtd_checkpoint_load(fdtd_handle h, const void *buf, size_t n);

@@ -271,10 +271,11 @@ static fdtd_div_plan div_plan_compute(float dx) {
   }
   /* scaling by 2^100 (quot_small in fdtd_flow.cu) takes every nonzero |a| < 1
    * to lo or above (2^-149 * 2^100 >= lo) and keeps a*2^100*y finite (y < 2^28;
-   * dx > 3.7e-9).  Otherwise such numerators are divided: on nanometre grids
-   * that costs time while a wave's front is in the CPML, where passing the
-   * numerator up to which the scaling holds to quot_small cost every grid: mode
-   * 5 4 % on 131x117x109, the others 1 %. */
+   * dx > 3.7e-9).  Otherwise such numerators are divided: from rest with dx =
+   * 1e-9 instead of 1e-8 that costs 2-24 % while the wave's front is in the CPML
+   * (176x160x129 mode 5 71 -> 86 us a step, separate kernels 96; 100^3 39 -> 49,
+   * 46), where passing the numerator up to which the scaling holds to quot_small
+   * cost every grid: 131x117x109 in mode 5 4 %, others 1 %. */
   p.small = p.lo <= 0x1p-60f && y < 0x1p28f;
   return p;
 }
@@ -1259,8 +1260,9 @@ static int autotune_zero_state(sim *s) {
 }
 
 /* The fused step: FDTD_FUSED=0 never, =1 always (no autotuning of the
- * choice), otherwise where the autotuner measures it faster (grids it
- * tunes).  Read at every ReadySimulation. */
+ * choice), otherwise, of the steps that multi-step launches do not take, where
+ * the autotuner measures it faster (grids it tunes, whatever their steps).
+ * Read at every ReadySimulation. */
 static int fused_mode(void) {
   const char *e = getenv("FDTD_FUSED");
   if (e && strcmp(e, "0") == 0) return 0;
